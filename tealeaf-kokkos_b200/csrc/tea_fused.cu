@@ -24,6 +24,7 @@
 #endif
 #include "../driver/tea_eigen.h"
 #include "tea_fused.cuh"
+#include "tea_resident.cuh"
 
 #define TEA_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -75,7 +76,22 @@ struct Fused {
     int stencil_mode = 0;  // 0: the faster kernel per sweep, 1: register pipeline only, 2: ring only
     Loop loops[LOOP_COUNT];
     bool use_graph = true;
+    // On-chip loops (tea_resident.cuh): the plans of an FP64 solve without and with the
+    // preconditioner and of the FP32 inner solves (blocks 0: the grid does not fit), the words
+    // the blocks exchange and the next unused epoch.
+    ResPlan res[2], res32;
+    ResWord* rim = nullptr;
+    unsigned long long* sums = nullptr;
+    unsigned long long epoch = 0;
+    int sum_set = 0;
 };
+
+// The solve state and, behind it, the failure flag of the on-chip loops, one allocation.
+constexpr size_t kStateBytes = (sizeof(SolveState) + 15) / 16 * 16 + 16;
+inline int* fail_of(SolveState* s)
+{
+    return reinterpret_cast<int*>(reinterpret_cast<char*>(s) + kStateBytes - 16);
+}
 
 Fused* fused_of(Chunk* c) { return static_cast<Fused*>(c->fused); }
 
@@ -379,6 +395,168 @@ void stencil(const Fused* F, const FusedArgs& a, cudaStream_t s)
     TEA_STENCIL<Op><<<F->stencil_blocks, TEA_STENCIL_BLOCK, 0, s>>>(a);
 }
 
+// The cheapest way to deal the grid to at most `sms` blocks, by a rough cost of one iteration in
+// nanoseconds: the row segments of the busiest warp, and with more than one block the waits for
+// the others and the halo cells.  blocks = 0 when no split fits.
+ResPlan res_plan(const Geom& g, int sms, int elem, bool pre, size_t smem)
+{
+    ResPlan best;
+    double best_cost = 0.0;
+    const int d3 = DIM == 3;
+    auto even = [](int n) { return (n + 1) / 2 * 2; };
+    const int xunits = (g.nx + 1) / 2;
+    for (int nbz = 1; nbz <= (d3 ? std::min(g.nz, sms) : 1); ++nbz)
+        for (int nby = 1; nby <= std::min(g.ny, sms / nbz); ++nby)
+            for (int nbx = 1; nbx <= std::min(xunits, sms / (nbz * nby)); ++nbx) {
+                ResPlan p;
+                p.blocks = nbx * nby * nbz;
+                p.nbx = nbx;
+                p.nby = nby;
+                p.nbz = nbz;
+                p.tw = std::min(g.nx, (xunits + nbx - 1) / nbx * 2);
+                p.th = (g.ny + nby - 1) / nby;
+                p.td = (g.nz + nbz - 1) / nbz;
+                // A strip's rows are dealt to as many warps as there are.
+                const long strips = (long)((p.tw + 63) / 64) * p.td;
+                int need = 0;
+                for (int form = 0; form < RES_FORM_COUNT; ++form) {
+                    const int warps = RES_FORMS[form].warps;
+                    if (strips > warps) continue;
+                    const int chunks = (int)std::min<long>(p.th, warps / strips);
+                    const int rows = (p.th + chunks - 1) / chunks;
+                    if (rows > RES_FORMS[form].rows) continue;
+                    need = rows;
+                    p.form = form;
+                    p.chunks = (p.th + rows - 1) / rows;
+                    break;
+                }
+                if (need == 0) continue;
+                p.warps = (int)strips * p.chunks;
+                if (p.blocks > 1 && p.warps < 2) p.warps = 2;
+                p.sx = even(p.tw + 4);
+                p.kxs = even(p.tw + 3);
+                p.tws = even(p.tw + 1);
+                p.halo = (nbx > 1 ? 2 * p.th * p.td : 0) + (nby > 1 ? 2 * p.tw * p.td : 0) + (nbz > 1 ? 2 * p.tw * p.th : 0);
+                p.pre = pre ? 1 : 0;
+                p.okx = (d3 ? p.td + 2 : 1) * (p.th + 2) * p.sx;
+                p.oky = p.okx + p.td * p.th * p.kxs;
+                p.okz = p.oky + p.td * (p.th + 1) * p.tws;
+                p.omi = p.okz + (d3 ? (p.td + 1) * p.th * p.tws : 0);
+                p.orh = p.omi + (pre ? p.td * p.th * p.tws : 0);
+                p.omh = p.orh + even(p.halo);
+                p.words = (p.omh + (pre ? even(p.halo) : 0) + 3) / 4 * 4;
+                p.bytes = (size_t)p.words * elem + (size_t)p.halo * sizeof(int2);
+                if (p.bytes > smem) continue;
+                const size_t own = (size_t)(p.td * p.th * p.tws + 3) / 4 * 4;
+                if (RES_FORMS[p.form].rows > 4 && p.bytes + own * elem <= smem) {
+                    p.ox = p.words;
+                    p.words += (int)own;
+                    p.bytes += own * elem;
+                }
+                const double cost =
+                    (p.form + 1 == RES_FORM_COUNT ? 600.0 : 300.0) * need * (0.4 + 0.6 * p.warps / RES_WARPS) +
+                    (p.blocks > 1 ? 1200.0 + 4.0 * p.blocks + 150.0 * p.halo / (32.0 * p.warps) : 0.0);
+                if (best.blocks == 0 || cost < best_cost) {
+                    best = p;
+                    best_cost = cost;
+                }
+            }
+    return best;
+}
+
+template <class K>
+void res_opt_in(K kernel, size_t bytes)
+{
+    TEA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
+// Plans of the on-chip loops and the words their blocks exchange (rim words only for grids
+// that fit: at most 33 MB).
+void setup_resident(Chunk* c, Fused* F, int sms)
+{
+    int optin = 0, coop = 0;
+    TEA_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
+    TEA_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
+    const size_t smem = optin > 2048 ? (size_t)optin - 2048 : 0;  // less the kernels' static part
+    if (!coop || (size_t)c->g.nx * c->g.ny * c->g.nz > (size_t)sms * RES_WARPS * 8 * 64) return;
+    F->res[0] = res_plan(c->g, sms, sizeof(double), false, smem);
+    F->res[1] = res_plan(c->g, sms, sizeof(double), true, smem);
+    F->res32 = res_plan(c->g, sms, sizeof(float), false, smem);
+    if (F->res[0].blocks == 0 && F->res32.blocks == 0) return;
+    const size_t rim = 2 * c->field_elems * sizeof(ResWord), sums = RES_SUM_WORDS * sizeof(unsigned long long);
+    TEA_CK(cudaMalloc(&F->rim, rim));
+    TEA_CK(cudaMalloc(&F->sums, sums));
+    if (!F->rim || !F->sums) {
+        F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;
+        return;
+    }
+    TEA_CK(cudaMemsetAsync(F->rim, 0, rim, c->stream));
+    TEA_CK(cudaMemsetAsync(F->sums, 0, sums, c->stream));
+}
+
+template <class P, int F>
+const void* res_kernel(int kind)
+{
+    constexpr int RS = RES_FORMS[F].rows, W = RES_FORMS[F].warps;
+    if constexpr (P::fp32) {
+        return kind == LOOP_CG32 ? (const void*)k_res_cg<P, RS, W> : (const void*)k_res_cheby<P, RS, W>;
+    } else {
+        switch (kind) {
+        case LOOP_CG: return (const void*)k_res_cg<P, RS, W>;
+        case LOOP_CHEBY: return (const void*)k_res_cheby<P, RS, W>;
+        case LOOP_PPCG: return (const void*)k_res_ppcg<P, RS, W>;
+        default: return (const void*)k_res_jacobi<P, RS, W>;
+        }
+    }
+}
+template <class P>
+const void* res_kernel(int kind, int form)
+{
+    static_assert(RES_FORM_COUNT == 5, "every form has its kernels");
+    switch (form) {
+    case 0: return res_kernel<P, 0>(kind);
+    case 1: return res_kernel<P, 1>(kind);
+    case 2: return res_kernel<P, 2>(kind);
+    case 3: return res_kernel<P, 3>(kind);
+    default: return res_kernel<P, 4>(kind);
+    }
+}
+
+// Launch loop `kind` as one on-chip kernel from the host's state; false when the grid, the loop
+// or the state is not of a form it takes (then the loop runs as a graph).
+bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
+{
+    const SolveState& s = *F->h_st;
+    const bool fp32 = kind == LOOP_CG32 || kind == LOOP_CHEBY32;
+    if (kind == LOOP_PPCG32 || (kind == LOOP_PPCG && s.precond)) return false;
+    const ResPlan& p = fp32 ? F->res32 : F->res[(kind == LOOP_CG || kind == LOOP_CHEBY) && s.precond ? 1 : 0];
+    if (p.blocks == 0 || s.par_u || s.par_p || s.pending_p || s.pending_u) return false;
+    ResArgs A;
+    A.f = F->base;
+    A.p = p;
+    A.s0 = s;
+    A.rim = F->rim;
+    A.elems = (long)c->field_elems;
+    A.sums = F->sums;
+    A.set = F->sum_set;
+    A.scale = kind == LOOP_CHEBY || kind == LOOP_JACOBI ? s.error : s.rro;
+    A.epoch = F->epoch;
+    A.fail = fail_of(F->d_st);
+    const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
+    res_opt_in(k, p.bytes);
+    void* args[] = {&A};
+    if (cudaLaunchCooperativeKernel(k, dim3(p.blocks), dim3(32 * p.warps), args, p.bytes, c->stream) != cudaSuccess) {
+        // Fewer SMs than the device reports (a partition of it): the loops run as graphs.
+        cudaGetLastError();
+        F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;
+        return false;
+    }
+    // More epochs than the loop can use: two rim exchanges and one per inner step an iteration.
+    F->epoch += (unsigned long long)(s.max_iters + 2) * (inner_steps + 4) + 16;
+    F->sum_set ^= 1;
+    return true;
+}
+
 Fused* ensure_fused(Chunk* c, int max_iters)
 {
     Fused* F = fused_of(c);
@@ -387,9 +565,9 @@ Fused* ensure_fused(Chunk* c, int max_iters)
         c->fused = F;
         const char* env = std::getenv("TEA_B200_NO_GRAPH");
         F->use_graph = !(env && env[0] == '1');
-        TEA_CK(cudaMalloc(&F->d_st, sizeof(SolveState)));
-        TEA_CK(cudaMemset(F->d_st, 0, sizeof(SolveState)));
-        TEA_CK(cudaHostAlloc(&F->h_st, sizeof(SolveState), cudaHostAllocDefault));
+        TEA_CK(cudaMalloc(&F->d_st, kStateBytes));
+        TEA_CK(cudaMemset(F->d_st, 0, kStateBytes));
+        TEA_CK(cudaHostAlloc(&F->h_st, kStateBytes, cudaHostAllocDefault));
         for (int k = 0; k < 3; ++k) {
             TEA_CK(cudaMalloc(&F->alt[k], c->field_elems * sizeof(double)));
             if (F->alt[k]) TEA_CK(cudaMemset(F->alt[k], 0, c->field_elems * sizeof(double)));
@@ -511,6 +689,7 @@ Fused* ensure_fused(Chunk* c, int max_iters)
             }
         }
 #endif
+        if (F->use_graph && F->stencil_mode == 0) setup_resident(c, F, sms);
         F->point_blocks = launch_blocks(c, c->inner.ntiles);
         {
             // Segment walks: at most one segment per warp, and at most one wave of the
@@ -784,8 +963,8 @@ void push_state(Chunk* c, Fused* F)
 
 void pull_state(Chunk* c, Fused* F)
 {
-    TEA_CK(cudaMemcpyAsync(F->h_st, F->d_st, sizeof(SolveState), cudaMemcpyDeviceToHost, c->stream));
-    c->d2h_bytes += sizeof(SolveState);
+    TEA_CK(cudaMemcpyAsync(F->h_st, F->d_st, kStateBytes, cudaMemcpyDeviceToHost, c->stream));
+    c->d2h_bytes += kStateBytes;
     sync(c);
 }
 
@@ -793,6 +972,15 @@ void pull_state(Chunk* c, Fused* F)
 void run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
 {
     F->h_st->cont = 1;  // the body runs at least once (the while node's default)
+    if (launch_resident(c, F, kind, inner_steps)) {
+        pull_state(c, F);
+        if (*fail_of(F->h_st)) {
+            set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of an on-chip loop lost one another");
+            TEA_CK(cudaMemsetAsync(fail_of(F->d_st), 0, sizeof(int), c->stream));
+            TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
+        }
+        return;
+    }
     push_state(c, F);
     if (F->use_graph && build_loop(c, F, kind, inner_steps)) {
         TEA_CK(cudaGraphLaunch(F->loops[kind].exec, c->stream));
@@ -888,6 +1076,8 @@ void destroy_fused(Chunk* c)
         if (p) cudaFree(p);
     for (float* p : F->alloc32)
         if (p) cudaFree(p);
+    if (F->rim) cudaFree(F->rim);
+    if (F->sums) cudaFree(F->sums);
     if (F->d_st) cudaFree(F->d_st);
     if (F->h_st) cudaFreeHost(F->h_st);
     delete F;

@@ -1,0 +1,1180 @@
+// On-chip iteration loops of the whole-solve path for grids that fit into the SMs' shared
+// memory and registers: one cooperative launch runs a whole loop (CG, Chebyshev, PPCG or
+// Jacobi, and the FP32 inner CG and Chebyshev solves) instead of a CUDA graph that launches
+// one or more kernels per iteration.
+//
+// What bounds it.  On such grids a launch is all latency: reading the state, filling the
+// row rings, the reduction's last block and the next launch take 6-12 us whatever the size,
+// two launches an iteration (20.6 us per CG iteration at 512^2).  Here one block per SM
+// owns a tile of the grid for the whole loop.  The stencil operand V (p, u or sd) sits in
+// shared memory with a one-cell halo, the face coefficients beside it, the other vectors
+// (r, w, p, u) in the registers of the threads that own the cells.  What is left of an
+// iteration is the arithmetic, one exchange of the tile's rim and the dot products.
+//
+// Work split.  A warp owns up to RS consecutive rows of a strip 64 cells wide (two cells per
+// lane), so that a row's y-neighbours and its lower face coefficient come from the registers
+// of the row before.  A block has 16 warps for up to four rows each, 12 (of 168 registers a
+// thread) for up to eight, and 16 again only where 12 are too few: beside 220 KB of shared
+// memory the L1 cache is too small for spills, and CG at 850^2 takes 7.6 us an iteration
+// with 12 warps and 12.0 with 16.  At the domain's faces a neighbour is the
+// cell itself, as the reference's reflecting halo update gives it; only the faces shared by
+// two tiles have halo cells.
+//
+// Exchange.  A rim value travels as one 16-byte word {value, epoch}: the owner stores it
+// with one 128-bit store, the reader polls the word until it carries the epoch it needs, so
+// no fence and no separate flag is needed.  Words are double-buffered by the epoch's parity:
+// a block can be at most one epoch ahead of a neighbour, because it needs that neighbour's
+// word of the same epoch to go on.
+//
+// Sums.  An all-to-all of the blocks' double-double partials through such words took 2400-2900
+// cycles at 64-128 blocks, a counter that all blocks add to and poll 1400-1550 (148 blocks),
+// so a dot product is formed by integer atomics: each thread's partial is cut into five 22-bit
+// limbs at bit positions that all blocks know (from the last value of the same sum), the
+// limbs add up exactly in any order, and each limb's 64-bit word counts its arrivals in
+// its top byte, so that the poll that sees the last arrival has the sum.  The integer sums
+// also replace five levels of double-double merges in a warp by five redux instructions.
+// Every block then forms the rounded value and runs the scalar recurrence and the loop test
+// itself.  A thread's partial is kept to 2^-89 of the sum's last value: rounded, the sums are
+// those of the per-launch kernels' double-double bit for bit, and per cell the operations and
+// their order are those of the per-call kernels.
+//
+// Every poll is bounded; a block that gives up raises a flag that ends the other blocks'
+// polls too, and the host reports the solve as failed.
+#pragma once
+
+#include <math_constants.h>
+
+#include "tea_fused.cuh"
+
+namespace tea {
+
+constexpr int RES_WARPS = 16;  // most warps of a block
+// The kernels' forms: at most RS rows a warp, W warps a block.
+struct ResForm {
+    int rows, warps;
+};
+constexpr ResForm RES_FORMS[] = {{1, 16}, {2, 16}, {4, 16}, {8, 12}, {8, 16}};
+constexpr int RES_FORM_COUNT = 5;
+constexpr int RES_POLLS = 1 << 21;  // rounds of polls before a wait gives up (a second or two)
+constexpr int RES_LIMBS = 5;         // limbs of a sum, and one word of flags
+constexpr int RES_SUM_STRIDE = 32;   // 64-bit words between two sums: a sum's words share a line
+constexpr int RES_SUM_WORDS = 2 * 2 * RES_SUM_STRIDE;  // two sets of two parities
+
+struct ResWord {
+    unsigned long long v, tag;
+};
+
+// How the grid is dealt to the blocks and a tile to the warps, and where things lie in shared
+// memory.
+struct ResPlan {
+    int blocks = 0;           // 0: the grid does not fit
+    int nbx = 1, nby = 1, nbz = 1;
+    int warps = 1, form = 0;  // warps of a block, kernel form
+    int tw = 0, th = 0, td = 0;  // largest tile
+    int chunks = 1;           // a strip's rows are dealt to this many warps
+    int sx = 0, kxs = 0, tws = 0;  // row strides of V, of Kx, and of the other arrays
+    int halo = 0;             // most halo cells of a tile
+    int pre = 0;              // with the preconditioner's diagonal
+    int okx = 0, oky = 0, okz = 0, omi = 0, orh = 0, omh = 0;  // first elements of Kx, Ky, Kz, mi, halo r, halo mi
+    int ox = 0;               // ... of one more vector of the loop, where there is room (else 0)
+    int words = 0;            // elements of T before the halo table
+    size_t bytes = 0;         // dynamic shared memory
+};
+
+struct ResArgs {
+    FusedArgs f;
+    ResPlan p;
+    SolveState s0;   // the state the loop starts from (the final one goes to *f.st)
+    ResWord* rim;    // [2][elems]: rim values by the cell's array index (from the allocation's start)
+    long elems;
+    unsigned long long* sums;  // RES_SUM_WORDS; this launch's set is zero, the other set's words
+    int set;                   // are cleared for the next launch
+    unsigned long long epoch;  // the rim exchanges' last epoch before this launch
+    double scale;              // expected magnitude of the sums
+    int* fail;
+};
+
+// First cell of part i of n parts of `cells` (in units of `unit` cells).
+__host__ __device__ inline int res_split(int cells, int unit, int i, int n)
+{
+    const int units = (cells + unit - 1) / unit;
+    const int c = (int)((long)i * units / n) * unit;
+    return c < cells ? c : cells;
+}
+
+// ------------------------------------------------------------------ words
+
+__device__ __forceinline__ void res_put(ResWord* p, unsigned long long v, unsigned long long tag)
+{
+    asm volatile("{\n .reg .b128 q;\n mov.b128 q, {%1, %2};\n st.relaxed.gpu.global.b128 [%0], q;\n}\n" ::"l"(p), "l"(v),
+                 "l"(tag)
+                 : "memory");
+}
+__device__ __forceinline__ ResWord res_get(const ResWord* p)
+{
+    ResWord w;
+    asm volatile("{\n .reg .b128 q;\n ld.relaxed.gpu.global.b128 q, [%2];\n mov.b128 {%0, %1}, q;\n}\n"
+                 : "=l"(w.v), "=l"(w.tag)
+                 : "l"(p)
+                 : "memory");
+    return w;
+}
+// The value of a word once it carries `tag`; after the poll limit, or when another block has
+// given up, sets gave_up and returns whatever is there.
+__device__ __forceinline__ unsigned long long res_wait(const ResWord* q, unsigned long long tag, int* fail, bool& gave_up)
+{
+    ResWord w = res_get(q);
+    for (int k = 0; w.tag != tag; ++k) {
+        if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)fail != 0)) {
+            gave_up = true;
+            break;
+        }
+        w = res_get(q);
+    }
+    return w.v;
+}
+__device__ __forceinline__ unsigned long long res_bits(double v) { return (unsigned long long)__double_as_longlong(v); }
+__device__ __forceinline__ unsigned long long res_bits(float v) { return (unsigned long long)__float_as_uint(v); }
+template <class T>
+__device__ __forceinline__ T res_value(unsigned long long b);
+template <>
+__device__ __forceinline__ double res_value<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
+template <>
+__device__ __forceinline__ float res_value<float>(unsigned long long b) { return __uint_as_float((unsigned)b); }
+
+// ------------------------------------------------------------------ sums
+
+// Limb positions of a sum, from the biased exponent E of its expected magnitude m: a thread's
+// partial may reach 2^8 m, the limbs are 22 bits apart (so that a block's total of a limb is
+// below 2^31), the first one's unit is 2^-13 m and the last one's 2^-101 m.
+constexpr int RES_E_MIN = 130, RES_E_MAX = 1980;  // expected exponents stay inside (units are normal numbers)
+constexpr int RES_E_UNIT = -13, RES_E_STEP = 22, RES_E_ROOM = 7;
+constexpr int RES_E_LOST = 10;  // a sum this far below the expected magnitude is formed again
+
+__device__ __forceinline__ int res_exponent(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+__device__ __forceinline__ int res_clamp(int e) { return min(max(e, RES_E_MIN), RES_E_MAX); }
+__device__ __forceinline__ double res_unit(int E, int limb)
+{
+    return __hiloint2double((E + RES_E_UNIT - RES_E_STEP * limb) << 20, 0);
+}
+
+// A lane's partial hi + lo cut into limbs: 1.5 * 2^52 units plus the rest has the limb in its
+// low word.  lo, below 2^-43 m, joins after the second limb, whose rest is below 2^-36 m: what
+// that sum rounds off is below 2^-89 m.
+__device__ __forceinline__ void res_limbs(double hi, double lo, int E, int (&v)[RES_LIMBS])
+{
+    double rest = hi;
+#pragma unroll
+    for (int i = 0; i < RES_LIMBS; ++i) {
+        const double cut = __hiloint2double(((E + RES_E_UNIT + 52 - RES_E_STEP * i) << 20) | 0x00080000, 0);
+        const double t = cut + rest;
+        v[i] = __double2loint(t);
+        rest = rest - (t - cut);
+        if (i == 1) rest = rest + lo;
+    }
+}
+
+// ------------------------------------------------------------------ a block's tile
+
+template <class T>
+struct alignas(2 * sizeof(T)) Two {
+    T x, y;
+};
+template <class T>
+__device__ __forceinline__ Two<T> ld_two(const T* p) { return *reinterpret_cast<const Two<T>*>(p); }
+template <class T>
+__device__ __forceinline__ void st_two(T* p, T x, T y)
+{
+    Two<T> v;
+    v.x = x;
+    v.y = y;
+    *reinterpret_cast<Two<T>*>(p) = v;
+}
+
+struct ResShared {
+    SolveState s;
+    int limbs[RES_LIMBS][RES_WARPS];
+    int scale[2];  // expected exponents of the loop's two sums
+    int bad;       // a partial out of range (1) or not finite (2)
+    int next;      // what follows a sum or an iteration: RN_*
+    double sum;    // the last sum
+};
+enum { RN_GO = 0, RN_STOP = 1, RN_AGAIN = 2, RN_FAIL = 4 };
+
+enum {
+    RF_A0 = 1, RF_A1 = 2,                // the lane's cells exist
+    RF_XM = 4, RF_XP0 = 8, RF_XP1 = 16,  // an x-neighbour is the cell itself (domain face)
+    RF_P0 = 32, RF_P1 = 64,              // the cells of every row lie on the tile's rim
+    RF_PFIRST = 128, RF_PLAST = 256,     // the first (last) row's do
+    RF_WFIRST = 512, RF_WLAST = 1024     // the row below the first (above the last) is itself
+};
+
+template <class T, int RS>
+struct ResTile {
+    const ResArgs& A;
+    const Geom& g;
+    ResShared& sh;
+    T* const V;   // shared memory: the operand, then the arrays at the plan's offsets
+    int nh;       // halo cells of this tile
+    int nw, warp, lane;
+    int x0, y0, z0, tw, th, td;  // first cell (0-based inner) and extents
+    int sx, plane;
+    // The warp's rows: y .. y + rows - 1 of plane z, columns x and x + 1 of this lane.
+    int rows, x, y, z;
+    int o, okx, oky, okz;  // offsets of the first row in V, Kx, Ky and Kz
+    long gi;               // its array index
+    int fl;                // RF_* flags
+    int dzm, dzp;          // offsets of the z-neighbours (0 at a domain face)
+    unsigned long long tag;   // epoch of the last rim exchange
+    unsigned long long seen0 = 0, seen1 = 0;  // this lane's word of the sums, as last read, by parity
+    int parity = 0;
+    bool gave_up = false;
+
+    __device__ __forceinline__ ResTile(const ResArgs& a, ResShared& s, T* mem) : A(a), g(a.f.g), sh(s), V(mem)
+    {
+        const ResPlan& p = a.p;
+        warp = threadIdx.x >> 5;
+        lane = threadIdx.x & 31;
+        nw = blockDim.x >> 5;
+        const int b = blockIdx.x;
+        const int bx = b % p.nbx, by = (b / p.nbx) % p.nby, bz = b / (p.nbx * p.nby);
+        x0 = res_split(g.nx, 2, bx, p.nbx);
+        tw = res_split(g.nx, 2, bx + 1, p.nbx) - x0;
+        y0 = res_split(g.ny, 1, by, p.nby);
+        th = res_split(g.ny, 1, by + 1, p.nby) - y0;
+        z0 = res_split(g.nz, 1, bz, p.nbz);
+        td = res_split(g.nz, 1, bz + 1, p.nbz) - z0;
+        sx = p.sx;
+        plane = (th + 2) * sx;
+        tag = a.epoch;
+        // The warp's strip, plane and rows.
+        const int strips = (tw + 63) / 64;
+        const int strip = warp % strips, rest = warp / strips;
+        const int chunk = rest % p.chunks;
+        z = rest / p.chunks;
+        y = res_split(th, 1, chunk, p.chunks);
+        rows = z < td ? res_split(th, 1, chunk + 1, p.chunks) - y : 0;
+        if (rows == 0) y = z = 0;
+        x = strip * 64 + 2 * lane;
+        const bool a0 = rows > 0 && x < tw, a1 = rows > 0 && x + 1 < tw;
+        const bool xl = x0 == 0, xr = x0 + tw == g.nx;
+        const bool zrim = (z == 0 && z0 > 0) || (z == td - 1 && z0 + td < g.nz);
+        fl = (a0 ? RF_A0 : 0) | (a1 ? RF_A1 : 0) | (x == 0 && xl ? RF_XM : 0) | (x == tw - 1 && xr ? RF_XP0 : 0) |
+             (x + 1 == tw - 1 && xr ? RF_XP1 : 0) |
+             (a0 && (zrim || (x == 0 && !xl) || (x == tw - 1 && !xr)) ? RF_P0 : 0) |
+             (a1 && (zrim || (x + 1 == tw - 1 && !xr)) ? RF_P1 : 0) | (y == 0 && y0 > 0 ? RF_PFIRST : 0) |
+             (y + rows == th && y0 + th < g.ny ? RF_PLAST : 0) | (y == 0 && y0 == 0 ? RF_WFIRST : 0) |
+             (y + rows == th && y0 + th == g.ny ? RF_WLAST : 0);
+        dzm = z == 0 && z0 == 0 ? 0 : plane;
+        dzp = z == td - 1 && z0 + td == g.nz ? 0 : plane;
+        const int row = z * th + y;
+        o = ((DIM == 3 ? (z + 1) * (th + 2) : 0) + y + 1) * sx + x + 2;
+        okx = p.okx + row * p.kxs + x;
+        oky = p.oky + (row + z) * p.tws + x;
+        okz = p.okz + row * p.tws + x;
+        gi = fidx(g, HALO_PAD + x0 + x, HALO_PAD + y0 + y, DIM == 3 ? HALO_PAD + z0 + z : 0);
+        build_table();
+    }
+
+    __device__ __forceinline__ bool on(int k) const { return (fl & RF_A0) && k < rows; }
+    __device__ __forceinline__ bool both() const { return fl & RF_A1; }
+    __device__ __forceinline__ long gidx(int k) const { return gi + k * g.pitch; }
+    __device__ __forceinline__ T* cell(int k) const { return V + o + k * sx; }
+    __device__ __forceinline__ Two<T> mi_of(int k) const { return ld_two(V + okz + (A.p.omi - A.p.okz) + k * A.p.tws); }
+    __device__ __forceinline__ T* own(int k) const { return V + okz + (A.p.ox - A.p.okz) + k * A.p.tws; }
+    __device__ __forceinline__ int2* table() const { return reinterpret_cast<int2*>(V + A.p.words); }  // halo cells: {offset in V, array index}
+    __device__ __forceinline__ T& halo_r(int h) const { return V[A.p.orh + h]; }
+    __device__ __forceinline__ T& halo_mi(int h) const { return V[A.p.omh + h]; }
+
+    // The tile's halo cells: the faces it shares with other tiles, without edges and corners.
+    __device__ void build_table()
+    {
+        const int fx = th * td, fy = tw * td, fz = DIM == 3 ? tw * th : 0;
+        const bool has[6] = {x0 > 0, x0 + tw < g.nx, y0 > 0, y0 + th < g.ny, DIM == 3 && z0 > 0, DIM == 3 && z0 + td < g.nz};
+        const int cnt[3] = {fx, fy, fz};
+        int base = 0;
+        for (int f = 0; f < 6; ++f) {
+            if (!has[f]) continue;
+            const int n = cnt[f >> 1];
+            for (int h = threadIdx.x; h < n; h += blockDim.x) {
+                int hx, hy, hz;
+                if (f < 2) {
+                    hx = f == 0 ? -1 : tw;
+                    hy = h % th;
+                    hz = h / th;
+                } else if (f < 4) {
+                    hy = f == 2 ? -1 : th;
+                    hx = h % tw;
+                    hz = h / tw;
+                } else {
+                    hz = f == 4 ? -1 : td;
+                    hx = h % tw;
+                    hy = h / tw;
+                }
+                const int vr = DIM == 3 ? (hz + 1) * (th + 2) + hy + 1 : hy + 1;
+                table()[base + h] = make_int2(vr * sx + hx + 2,
+                                            (int)fidx(g, HALO_PAD + x0 + hx, HALO_PAD + y0 + hy,
+                                                      DIM == 3 ? HALO_PAD + z0 + hz : 0));
+            }
+            base += n;
+        }
+        nh = base;
+    }
+
+    // Fill the coefficient arrays from the fields (mi in a preconditioned solve, else null).
+    __device__ void load_coefs(const T* kx, const T* ky, const T* kz, const T* mi)
+    {
+        T *KX = V + A.p.okx, *KY = V + A.p.oky, *KZ = V + A.p.okz, *MI = V + A.p.omi;
+        for (int r = warp; r < th * td; r += nw) {
+            const int rz = r / th, ry = r - rz * th;
+            const long i = fidx(g, HALO_PAD + x0, HALO_PAD + y0 + ry, DIM == 3 ? HALO_PAD + z0 + rz : 0);
+            for (int c = lane; c <= tw; c += 32) KX[r * A.p.kxs + c] = kx[i + c];
+            for (int c = lane; c < tw; c += 32) {
+                KY[(r + rz) * A.p.tws + c] = ky[i + c];
+                if (ry == th - 1) KY[(r + rz + 1) * A.p.tws + c] = ky[i + g.pitch + c];
+                if (DIM == 3) {
+                    KZ[r * A.p.tws + c] = kz[i + c];
+                    if (rz == td - 1) KZ[(r + th) * A.p.tws + c] = kz[i + g.page + c];
+                }
+                if (mi) MI[r * A.p.tws + c] = mi[i + c];
+            }
+        }
+    }
+    // V and its halo from a field.
+    __device__ void load_operand(const T* v)
+    {
+        for (int r = warp; r < th * td; r += nw) {
+            const int rz = r / th, ry = r - rz * th;
+            const long i = fidx(g, HALO_PAD + x0, HALO_PAD + y0 + ry, DIM == 3 ? HALO_PAD + z0 + rz : 0);
+            const int vr = DIM == 3 ? (rz + 1) * (th + 2) + ry + 1 : ry + 1;
+            for (int c = lane; c < tw; c += 32) V[vr * sx + c + 2] = v[i + c];
+        }
+        __syncthreads();  // the table
+        for (int h = threadIdx.x; h < nh; h += blockDim.x) V[table()[h].x] = v[table()[h].y];
+    }
+    __device__ void load_halo_mi(const T* mi)
+    {
+        for (int h = threadIdx.x; h < nh; h += blockDim.x) halo_mi(h) = mi[table()[h].y];
+    }
+
+    // The operator's operands at the warp's rows in order: f(k, cell, nb, kx0, kx1, ky0, ky1,
+    // kz0, kz1) for the two cells of each row.
+    template <class F>
+    __device__ __forceinline__ void sweep(F&& f) const
+    {
+        if (!(fl & RF_A0)) return;
+        Two<T> ym = ld_two(V + o - ((fl & RF_WFIRST) ? 0 : sx)), c = ld_two(V + o), ky0 = ld_two(V + oky);
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (k < rows) {
+                const T* vk = cell(k);
+                const Two<T> yp = ld_two(vk + (k == rows - 1 && (fl & RF_WLAST) ? 0 : sx));
+                const T l = vk[-1], r = vk[2];
+                const T* kxp = V + okx + k * A.p.kxs;
+                const Two<T> kx = ld_two(kxp);
+                const T kx2 = kxp[2];
+                const Two<T> ky1 = ld_two(V + oky + (k + 1) * A.p.tws);
+                Two<T> zm = c, zp = c, kz0, kz1;
+                kz0.x = kz0.y = kz1.x = kz1.y = (T)0;
+                if (DIM == 3) {
+                    zm = ld_two(vk - dzm);
+                    zp = ld_two(vk + dzp);
+                    kz0 = ld_two(V + okz + k * A.p.tws);
+                    kz1 = ld_two(V + okz + (k + th) * A.p.tws);
+                }
+                NbT<T> nb;
+                nb.c = c.x;
+                nb.xm = (fl & RF_XM) ? c.x : l;
+                nb.xp = (fl & RF_XP0) ? c.x : c.y;
+                nb.ym = ym.x;
+                nb.yp = yp.x;
+                nb.zm = zm.x;
+                nb.zp = zp.x;
+                f(k, 0, nb, kx.x, kx.y, ky0.x, ky1.x, kz0.x, kz1.x);
+                nb.c = c.y;
+                nb.xm = c.x;
+                nb.xp = (fl & RF_XP1) ? c.y : r;
+                nb.ym = ym.y;
+                nb.yp = yp.y;
+                nb.zm = zm.y;
+                nb.zp = zp.y;
+                f(k, 1, nb, kx.y, kx2, ky0.y, ky1.y, kz0.y, kz1.y);
+                ym = c;
+                c = yp;
+                ky0 = ky1;
+            }
+    }
+    // Adds a product to a thread's sum; the second cell of a row may not exist.
+    __device__ __forceinline__ void add(DD& acc, int q, double v) const { dd_add(acc, q == 0 || both() ? v : 0.0); }
+
+    __device__ __forceinline__ void store(int k, T v0, T v1) const
+    {
+        // The second cell of a lane past the tile's edge may be a halo cell.
+        if (both()) st_two(cell(k), v0, v1);
+        else *cell(k) = v0;
+    }
+    // Publish the rim cells of row k under the current exchange's epoch.
+    __device__ __forceinline__ void publish(int k, T v0, T v1) const
+    {
+        int rim = fl & (RF_P0 | RF_P1);
+        if ((k == 0 && (fl & RF_PFIRST)) || (k == rows - 1 && (fl & RF_PLAST))) rim = RF_P0 | (both() ? RF_P1 : 0);
+        if (rim) {
+            ResWord* q = A.rim + (tag & 1) * A.elems + kLeadPad + gidx(k);
+            if (rim & RF_P0) res_put(q, res_bits(v0), tag);
+            if (rim & RF_P1) res_put(q + 1, res_bits(v1), tag);
+        }
+    }
+    // The neighbours' values of the current exchange, through put(h, value); the warps from
+    // `first` on share the halo cells.
+    template <class F>
+    __device__ __forceinline__ void collect(int first, F&& put)
+    {
+        if (nh == 0 || warp < first) return;
+        const ResWord* q = A.rim + (tag & 1) * A.elems + kLeadPad;
+        for (int h = (warp - first) * 32 + lane; h < nh; h += (nw - first) * 32) {
+            put(h, res_value<T>(res_wait(q + table()[h].y, tag, A.fail, gave_up)));
+        }
+    }
+
+    // Sum number `which` of the loop over all blocks.  `meanwhile` runs in the other warps while
+    // warp 0 waits.  With the rounded sum, `control` runs in warp 0's first lane before any
+    // thread goes on (it returns whether the loop goes on), and `after` in the last warp's first
+    // lane while the others go on.  Returns RN_GO, RN_STOP or RN_FAIL.
+    template <class M, class C, class N>
+    __device__ __forceinline__ int reduce(const DD& acc, int which, M&& meanwhile, C&& control, N&& after)
+    {
+        for (int tries = 0;; ++tries) {
+            const int E = sh.scale[which];
+            double hi = acc.hi, lo = acc.lo;
+            if (res_exponent(hi) > E + RES_E_ROOM) {
+                atomicOr(&sh.bad, isfinite(hi) ? 1 : 2);
+                hi = lo = 0.0;
+            }
+            int v[RES_LIMBS];
+            res_limbs(hi, lo, E, v);
+#pragma unroll
+            for (int i = 0; i < RES_LIMBS; ++i) v[i] = __reduce_add_sync(0xffffffffu, v[i]);
+            if (lane == 0) {
+#pragma unroll
+                for (int i = 0; i < RES_LIMBS; ++i) sh.limbs[i][warp] = v[i];
+            }
+            parity ^= 1;
+            __syncthreads();
+            if (warp == 0) {
+                long long mine = 0;
+#pragma unroll
+                for (int i = 0; i < RES_LIMBS; ++i) {
+                    const int w = __reduce_add_sync(0xffffffffu, lane < nw ? sh.limbs[i][lane] : 0);
+                    if (lane == i) mine = w;
+                }
+                unsigned bad = sh.bad;
+                const int nb = A.p.blocks;
+                if (nb > 1) {
+                    // A count in the top byte; below it the limb, raised to be positive.  The warp
+                    // stays together: a lane that polled before another has added would wait
+                    // for a word that the other blocks' same lanes wait for too.  The atomics
+                    // return a value so that the polls begin when this block's have arrived
+                    // (1550 cycles a sum against 2050 at 64 blocks).
+                    constexpr long long bias = 1ll << 32;
+                    const bool has = lane <= RES_LIMBS;
+                    mine = lane == RES_LIMBS ? (long long)((bad & 1) + ((bad & 2) << 15)) : mine;
+                    unsigned long long* q =
+                        A.sums + (A.set * 2 + parity) * RES_SUM_STRIDE + (has ? lane : RES_LIMBS);
+                    const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + bias);
+                    const unsigned long long old = parity ? seen1 : seen0;
+                    unsigned long long now = old;
+                    if (has) asm volatile("atom.relaxed.gpu.global.add.u64 %0, [%1], %2;" : "=l"(now) : "l"(q), "l"(add) : "memory");
+                    __syncwarp();
+                    now += add;
+                    for (int k = 0; __any_sync(0xffffffffu, has && (int)((now - old) >> 56) != nb); ++k) {
+                        if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)A.fail != 0)) {
+                            gave_up = true;
+                            break;
+                        }
+                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(q) : "memory");
+                    }
+                    mine = (long long)((now - old) & ((1ull << 56) - 1)) - nb * bias;
+                    seen0 = parity ? seen0 : now;
+                    seen1 = parity ? now : seen1;
+                    bad = (unsigned)__shfl_sync(0xffffffffu, (int)mine, RES_LIMBS);
+                    bad = ((bad & 0xffff) ? 1 : 0) | ((bad >> 16) ? 2 : 0);
+                }
+                const double part = (double)mine * res_unit(E, lane < RES_LIMBS ? lane : 0);
+                DD s = {part, 0.0};
+#pragma unroll
+                for (int i = 1; i < RES_LIMBS; ++i) dd_add(s, __shfl_sync(0xffffffffu, part, i));
+                if (lane == 0) {
+                    double sum = dd_value(s);
+                    int e = res_clamp(res_exponent(sum)), next = RN_GO;
+                    if (bad & 2) {
+                        sum = CUDART_NAN;
+                        e = E;
+                    } else if (bad) {
+                        if (E == RES_E_MAX) sum = CUDART_INF;
+                        else next = RN_AGAIN;
+                        e = min(E + 2 * RES_E_ROOM * (tries + 1), RES_E_MAX);
+                    } else if (sum == 0.0) {
+                        e = E;
+                    } else if (e < E - RES_E_LOST) {
+                        next = RN_AGAIN;
+                    }
+                    if (next == RN_GO && !control(sum)) next = RN_STOP;
+                    sh.scale[which] = e;
+                    sh.sum = sum;
+                    sh.bad = 0;
+                    sh.next = next;
+                }
+            }
+            if (tries == 0) meanwhile();
+            const int next = finish();
+            if (next & RN_FAIL) return RN_FAIL;
+            if (!(next & RN_AGAIN)) {
+                if (threadIdx.x == 32 * (nw - 1)) after(sh.sum);
+                return next;
+            }
+        }
+    }
+    // The end of an exchange: after it every thread sees what the others have written and what
+    // warp 0 has decided.
+    __device__ __forceinline__ int finish()
+    {
+        if (gave_up) *(volatile int*)A.fail = 1;
+        return __syncthreads_or(gave_up) ? RN_FAIL : sh.next;
+    }
+};
+
+// Arrays of the FP64 solve and of the FP32 inner solves.
+struct ResF64 {
+    using T = double;
+    static constexpr bool fp32 = false;
+    __device__ static T* r(const FusedArgs& a) { return a.r; }
+    __device__ static T* w(const FusedArgs& a) { return a.w; }
+    __device__ static T* p(const FusedArgs& a) { return a.p[0]; }
+    __device__ static T* u(const FusedArgs& a) { return a.u[0]; }
+    __device__ static T* rhs(const FusedArgs& a) { return a.u0; }
+    __device__ static const T* kx(const FusedArgs& a) { return a.kx; }
+    __device__ static const T* ky(const FusedArgs& a) { return a.ky; }
+    __device__ static const T* kz(const FusedArgs& a) { return a.kz; }
+    __device__ static const T* mi(const FusedArgs& a, bool pre) { return pre ? a.mi : nullptr; }
+};
+struct ResF32 {
+    using T = float;
+    static constexpr bool fp32 = true;
+    __device__ static T* r(const FusedArgs& a) { return a.r32; }
+    __device__ static T* w(const FusedArgs& a) { return a.w32; }
+    __device__ static T* p(const FusedArgs& a) { return a.p32[0]; }
+    __device__ static T* u(const FusedArgs& a) { return a.d32; }
+    __device__ static T* rhs(const FusedArgs& a) { return a.r32; }
+    __device__ static const T* kx(const FusedArgs& a) { return a.kx32; }
+    __device__ static const T* ky(const FusedArgs& a) { return a.ky32; }
+    __device__ static const T* kz(const FusedArgs& a) { return a.kz32; }
+    __device__ static const T* mi(const FusedArgs&, bool) { return nullptr; }
+};
+
+// A lane's two cells of an array (rows are padded, so the pair is always inside it).
+template <class T>
+__device__ __forceinline__ void ld_cells(const T* a, long i, T& x, T& y)
+{
+    const Two<T> v = ld_two(a + i);
+    x = v.x;
+    y = v.y;
+}
+template <class T>
+__device__ __forceinline__ void st_cells(T* a, long i, bool both, T x, T y)
+{
+    if (both) st_two(a + i, x, y);
+    else a[i] = x;
+}
+
+// A vector that the loop reads (or updates) at a warp's own cells only: u, or the right-hand
+// side.  Up to four rows of it stay in registers; with more rows the two vectors that are live
+// across a sum fill the registers, and it lies in shared memory where there is room, else in
+// L2, from which all rows are loaded before any is stored.
+template <class T, int RS>
+struct ResOwn {
+    static constexpr bool kept = RS * sizeof(T) <= 32;
+    T v[kept ? RS : 1][2];
+    T* far;  // the array
+    __device__ __forceinline__ ResOwn(const ResTile<T, RS>& t, T* array) : far(array)
+    {
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                if constexpr (kept) {
+                    ld_cells(far, t.gidx(k), v[k][0], v[k][1]);
+                } else if (t.A.p.ox) {
+                    const Two<T> c = ld_two(far + t.gidx(k));
+                    st_two(t.own(k), c.x, c.y);
+                }
+            }
+    }
+    // The rows, in `w` when they are not kept.
+    __device__ __forceinline__ void load(const ResTile<T, RS>& t, T (&w)[RS][2]) const
+    {
+        if constexpr (kept) {
+#pragma unroll
+            for (int k = 0; k < RS; ++k) {
+                w[k][0] = v[k][0];
+                w[k][1] = v[k][1];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) {
+                    const Two<T> c = ld_two(t.A.p.ox ? t.own(k) : far + t.gidx(k));
+                    w[k][0] = c.x;
+                    w[k][1] = c.y;
+                }
+        }
+    }
+    __device__ __forceinline__ void store(const ResTile<T, RS>& t, const T (&w)[RS][2])
+    {
+        if constexpr (kept) {
+#pragma unroll
+            for (int k = 0; k < RS; ++k) {
+                v[k][0] = w[k][0];
+                v[k][1] = w[k][1];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) {
+                    if (t.A.p.ox) st_two(t.own(k), w[k][0], w[k][1]);
+                    else st_cells(far, t.gidx(k), t.both(), w[k][0], w[k][1]);
+                }
+        }
+    }
+    // Back to the array at the end of a loop that updates it.
+    __device__ __forceinline__ void write(const ResTile<T, RS>& t) const
+    {
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                if constexpr (kept) {
+                    st_cells(far, t.gidx(k), t.both(), v[k][0], v[k][1]);
+                } else if (t.A.p.ox) {
+                    const Two<T> c = ld_two(t.own(k));
+                    st_cells(far, t.gidx(k), t.both(), c.x, c.y);
+                }
+            }
+    }
+};
+
+// The operator's diagonal at a cell, and the operator with it given: smvp_k's expression.
+template <class T>
+__device__ __forceinline__ T res_diag(T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
+{
+#if TEA_DIM == 2
+    (void)kz0;
+    (void)kz1;
+    return (T)1 + (kx1 + kx0) + (ky1 + ky0);
+#else
+    return (T)1 + (kx1 + kx0) + (ky1 + ky0) + (kz1 + kz0);
+#endif
+}
+template <class T>
+__device__ __forceinline__ T res_smvp(T d, const NbT<T>& a, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
+{
+#if TEA_DIM == 2
+    (void)kz0;
+    (void)kz1;
+    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym);
+#else
+    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym) - (kz1 * a.zp + kz0 * a.zm);
+#endif
+}
+
+// Diagonals of the warp's cells: in registers where there is room, else formed again from the
+// coefficients (four of the thirteen operations of the 2D operator).
+template <class T, int RS>
+struct ResDiag {
+    static constexpr bool kept = RS * sizeof(T) <= 16;
+    T d[kept ? RS : 1][2];
+    __device__ __forceinline__ void load(const ResTile<T, RS>& t)
+    {
+        if constexpr (kept)
+            t.sweep([&](int k, int q, const NbT<T>&, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+                d[k][q] = res_diag(kx0, kx1, ky0, ky1, kz0, kz1);
+            });
+    }
+    __device__ __forceinline__ T smvp(int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) const
+    {
+        if constexpr (kept) return res_smvp(d[k][q], nb, kx0, kx1, ky0, ky1, kz0, kz1);
+        else return smvp_k(nb, kx0, kx1, ky0, ky1, kz0, kz1);
+    }
+};
+
+#define RES_PROLOGUE(P)                                                                            \
+    using T = typename P::T;                                                                       \
+    extern __shared__ __align__(16) unsigned char s_res_raw[];                                     \
+    __shared__ ResShared sh;                                                                       \
+    const FusedArgs& a = A.f;                                                                      \
+    if (threadIdx.x == 0) {                                                                        \
+        sh.s = A.s0;                                                                               \
+        sh.scale[0] = sh.scale[1] = res_clamp(res_exponent(A.scale));                              \
+        sh.bad = 0;                                                                                \
+        sh.next = RN_GO;                                                                           \
+    }                                                                                              \
+    ResTile<T, RS> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                      \
+    ResDiag<T, RS> dg;                                                                             \
+    SolveState& s = sh.s
+
+#define RES_EPILOGUE()                                                                             \
+    __syncthreads();                                                                               \
+    if (blockIdx.x == 0) {                                                                         \
+        if (threadIdx.x == 0) *a.st = s;                                                           \
+        for (int i = threadIdx.x; i < RES_SUM_WORDS / 2; i += blockDim.x)                          \
+            A.sums[(A.set ^ 1) * (RES_SUM_WORDS / 2) + i] = 0;                                     \
+    }
+
+// CG: per iteration p = beta p + (z|r), w = A p and p.w; u += alpha p, r -= alpha w and
+// r.(r|z).  The neighbours' r arrives while the second sum is formed, and the halo of p follows
+// by the same recurrence, so an iteration waits for two sums and nothing else.
+template <class P, int RS, int W>
+__global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ ResArgs A)
+{
+    RES_PROLOGUE(P);
+    const bool pre = !P::fp32 && A.p.pre;
+    t.load_coefs(P::kx(a), P::ky(a), P::kz(a), P::mi(a, pre));
+    t.load_operand(P::p(a));
+    if (pre) t.load_halo_mi(P::mi(a, pre));
+    T r[RS][2], w[RS][2];
+    ResOwn<T, RS> u(t, P::u(a));
+#pragma unroll
+    for (int k = 0; k < RS; ++k) {
+        r[k][0] = r[k][1] = w[k][0] = w[k][1] = (T)0;
+        if (t.on(k)) ld_cells(P::r(a), t.gidx(k), r[k][0], r[k][1]);
+    }
+    __syncthreads();
+    dg.load(t);
+    for (bool pend = false;; pend = true) {
+        if (pend) {
+            const T beta = (T)s.last_beta;
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) {
+                    const Two<T> c = ld_two(t.cell(k));
+                    T q0 = r[k][0], q1 = r[k][1];
+                    if (pre) {
+                        const Two<T> m = t.mi_of(k);
+                        q0 = m.x * q0;
+                        q1 = m.y * q1;
+                    }
+                    t.store(k, beta * c.x + q0, beta * c.y + q1);
+                }
+            for (int h = threadIdx.x; h < t.nh; h += blockDim.x) {
+                T q = t.halo_r(h);
+                if (pre) q = t.halo_mi(h) * q;
+                T* c = t.V + t.table()[h].x;
+                *c = beta * *c + q;
+            }
+            __syncthreads();
+        }
+        DD acc = {0.0, 0.0};
+        t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+            const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+            w[k][q] = wv;
+            t.add(acc, q, (double)wv * (double)nb.c);
+        });
+        if (t.reduce(
+                acc, 0, [] {},
+                [&](double v) {
+                    s.alpha = s.rro / v;
+                    return true;
+                },
+                [&](double v) {
+                    s.pw = v;
+                    if (!P::fp32 && blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
+                    if (!isfinite(v)) s.nonfinite = 1;
+                }) != RN_GO)
+            break;
+        const T alpha = (T)s.alpha;
+        acc.hi = acc.lo = 0.0;
+        ++t.tag;
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                r[k][0] = r[k][0] - alpha * w[k][0];
+                r[k][1] = r[k][1] - alpha * w[k][1];
+                t.publish(k, r[k][0], r[k][1]);
+            }
+        // w is free: it takes u.
+        u.load(t, w);
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                const Two<T> c = ld_two(t.cell(k));
+                T q0 = r[k][0], q1 = r[k][1];
+                if (pre) {
+                    const Two<T> m = t.mi_of(k);
+                    q0 = m.x * q0;
+                    q1 = m.y * q1;
+                }
+                t.add(acc, 0, (double)r[k][0] * (double)q0);
+                t.add(acc, 1, (double)r[k][1] * (double)q1);
+                w[k][0] = w[k][0] + alpha * c.x;
+                w[k][1] = w[k][1] + alpha * c.y;
+            }
+        u.store(t, w);
+        const int next = t.reduce(
+            acc, 1, [&] { t.collect(1, [&](int h, T v) { t.halo_r(h) = v; }); },
+            [&](double v) {
+                s.last_beta = v / s.rro;
+                s.rro = v;
+                if constexpr (P::fp32) {
+                    const int n = ++s.n_inner;
+                    const bool at_switch = s.switch_err > 0.0 && n >= s.switch_min && v <= s.switch_err;
+                    s.cont = isfinite(v) && v >= s.tol2 && n < s.inner_max && !at_switch;
+                } else {
+                    s.error = v;
+                    end_iteration(a, s, PHASE_CG);
+                }
+                return s.cont != 0;
+            },
+            [&](double v) {
+                // The iteration that has just ended: end_iteration steps n unless it converged.
+                const int n = P::fp32 ? s.n_inner : (s.exit_reason == EXIT_CONVERGED ? s.n : s.n - 1);
+                s.rrn = v;
+                s.beta = s.last_beta;
+                s.last_alpha = s.alpha;
+                if (!isfinite(v)) s.nonfinite = 1;
+                if (blockIdx.x == 0) {
+                    if (P::fp32) a.cg_alphas[n] = s.alpha;
+                    a.cg_betas[n] = s.beta;
+                }
+            });
+        if (next != RN_GO) break;
+    }
+    __syncthreads();  // what the last sum left to be written down
+    t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+        w[k][q] = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+    });
+    if (threadIdx.x == 0) s.pending_p = 1;
+#pragma unroll
+    for (int k = 0; k < RS; ++k)
+        if (t.on(k)) {
+            const long i = t.gidx(k);
+            const Two<T> c = ld_two(t.cell(k));
+            st_cells(P::p(a), i, t.both(), c.x, c.y);
+            st_cells(P::r(a), i, t.both(), r[k][0], r[k][1]);
+            st_cells(P::w(a), i, t.both(), w[k][0], w[k][1]);
+            if constexpr (!P::fp32)
+                if (pre) {
+                    const Two<T> m = t.mi_of(k);
+                    st_cells(a.z, i, t.both(), m.x * r[k][0], m.y * r[k][1]);
+                }
+        }
+    u.write(t);
+    RES_EPILOGUE();
+}
+
+// Chebyshev: r = rhs - A u, p = alpha p + beta (mi r | r), u += p.  Iterations between two
+// checks only exchange the rim of u with the neighbouring tiles; r.r is summed where the loop
+// checks it.
+template <class P, int RS, int W>
+__global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__ ResArgs A)
+{
+    RES_PROLOGUE(P);
+    const bool pre = !P::fp32 && A.p.pre;
+    t.load_coefs(P::kx(a), P::ky(a), P::kz(a), P::mi(a, pre));
+    t.load_operand(P::u(a));
+    T p[RS][2], un[RS][2];
+    const ResOwn<T, RS> b(t, P::rhs(a));
+#pragma unroll
+    for (int k = 0; k < RS; ++k) {
+        p[k][0] = p[k][1] = un[k][0] = un[k][1] = (T)0;
+        if (t.on(k)) ld_cells(P::p(a), t.gidx(k), p[k][0], p[k][1]);
+    }
+    __syncthreads();
+    dg.load(t);
+    for (;;) {
+        const int step = P::fp32 ? s.n_inner - 1 : s.cheby_calc_steps - 1;
+        const T al = (T)a.ch_alphas[step], be = (T)a.ch_betas[step];
+        const bool check = P::fp32 ? s.n_inner % 10 == 0 : (s.n >= s.est_itc && s.n % 10 == 0);
+        DD acc = {0.0, 0.0};
+        ++t.tag;
+        Two<T> m;
+        m.x = m.y = (T)1;
+        b.load(t, un);
+        t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+            if (q == 0 && pre) m = t.mi_of(k);
+            const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+            const T rv = un[k][q] - wv;
+            const T pv = al * p[k][q] + be * (pre ? (q == 0 ? m.x : m.y) * rv : rv);
+            p[k][q] = pv;
+            un[k][q] = nb.c + pv;
+            if (check) t.add(acc, q, (double)rv * (double)rv);
+        });
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) t.publish(k, un[k][0], un[k][1]);
+        __syncthreads();  // every warp has read the old operand and the state
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) t.store(k, un[k][0], un[k][1]);
+        auto halo = [&](int first) { t.collect(first, [&](int h, T v) { t.V[t.table()[h].x] = v; }); };
+        auto finish = [&](double v) {
+            if constexpr (P::fp32) {
+                s.n_inner = s.n_inner + 1;
+                OpCheby32::finish(a, s, check, v);
+            } else {
+                if (check) s.error = v;
+                s.cheby_calc_steps = s.cheby_calc_steps + 1;
+                end_iteration(a, s, PHASE_CHEBY);
+            }
+            return s.cont != 0;
+        };
+        int next;
+        if (check) {
+            next = t.reduce(acc, 0, [&] { halo(t.nw > 1 ? 1 : 0); }, finish, [](double) {});
+        } else {
+            if (threadIdx.x == 0) sh.next = finish(0.0) ? RN_GO : RN_STOP;
+            halo(0);
+            next = t.finish();
+        }
+        if (next != RN_GO) break;
+    }
+#pragma unroll
+    for (int k = 0; k < RS; ++k)
+        if (t.on(k)) {
+            st_cells(P::u(a), t.gidx(k), t.both(), un[k][0], un[k][1]);
+            st_cells(P::p(a), t.gidx(k), t.both(), p[k][0], p[k][1]);
+        }
+    RES_EPILOGUE();
+}
+
+// PPCG without the preconditioner: the CG sweep on p, then the inner steps on sd, each with
+// one rim exchange; V holds p and then sd.
+template <class P, int RS, int W>
+__global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ ResArgs A)
+{
+    RES_PROLOGUE(P);
+    t.load_coefs(a.kx, a.ky, a.kz, nullptr);
+    t.load_operand(a.p[0]);
+    constexpr bool PREG = RS <= 2;  // p waits in registers, else in its array, for the next outer iteration
+    T r[RS][2], w[RS][2], p[PREG ? RS : 1][2];
+    ResOwn<T, RS> u(t, a.u[0]);
+#pragma unroll
+    for (int k = 0; k < RS; ++k) {
+        r[k][0] = r[k][1] = w[k][0] = w[k][1] = (T)0;
+        if (t.on(k)) {
+            ld_cells(a.r, t.gidx(k), r[k][0], r[k][1]);
+            if constexpr (PREG) ld_cells(a.p[0], t.gidx(k), p[k][0], p[k][1]);
+        }
+    }
+    auto set_operand = [&](int k, T v0, T v1) {
+        t.store(k, v0, v1);
+        t.publish(k, v0, v1);
+    };
+    auto exchange = [&] {
+        t.collect(0, [&](int h, T v) { t.V[t.table()[h].x] = v; });
+        return t.finish();
+    };
+    __syncthreads();
+    dg.load(t);
+    const int inner = s.inner_steps;
+    bool lost = false;
+    for (bool pend = false;; pend = true) {
+        if (pend) {
+            const T beta = s.last_beta;
+            ++t.tag;
+            if constexpr (PREG) {
+#pragma unroll
+                for (int k = 0; k < RS; ++k) {
+                    w[k][0] = p[k][0];
+                    w[k][1] = p[k][1];
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < RS; ++k)
+                    if (t.on(k)) ld_cells(a.p[0], t.gidx(k), w[k][0], w[k][1]);
+            }
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) {
+                    w[k][0] = beta * w[k][0] + r[k][0];
+                    w[k][1] = beta * w[k][1] + r[k][1];
+                    set_operand(k, w[k][0], w[k][1]);
+                    if constexpr (PREG) {
+                        p[k][0] = w[k][0];
+                        p[k][1] = w[k][1];
+                    } else {
+                        st_cells(a.p[0], t.gidx(k), t.both(), w[k][0], w[k][1]);
+                    }
+                }
+            if (exchange() != RN_GO) break;
+        }
+        DD acc = {0.0, 0.0};
+        t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+            const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+            w[k][q] = wv;
+            t.add(acc, q, wv * nb.c);
+        });
+        if (t.reduce(
+                acc, 0, [] {},
+                [&](double v) {
+                    s.alpha = s.rro / v;
+                    return true;
+                },
+                [&](double v) {
+                    s.pw = v;
+                    if (blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
+                    if (!isfinite(v)) s.nonfinite = 1;
+                }) != RN_GO)
+            break;
+        const T alpha = s.alpha, theta = s.theta;
+        ++t.tag;
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                r[k][0] = r[k][0] - alpha * w[k][0];
+                r[k][1] = r[k][1] - alpha * w[k][1];
+            }
+        u.load(t, w);
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                const Two<T> c = ld_two(t.cell(k));
+                w[k][0] = w[k][0] + alpha * c.x;
+                w[k][1] = w[k][1] + alpha * c.y;
+            }
+        u.store(t, w);
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) set_operand(k, r[k][0] / theta, r[k][1] / theta);
+        if (exchange() != RN_GO) break;
+        acc.hi = acc.lo = 0.0;
+        for (int m = 1; m <= inner; ++m) {
+            const T al = a.ch_alphas[m - 1], be = a.ch_betas[m - 1];
+            const bool last = m == inner;
+            // u += sd first: its rows pass through w, which then takes the new sd.
+            u.load(t, w);
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) {
+                    const Two<T> c = ld_two(t.cell(k));
+                    w[k][0] = w[k][0] + c.x;
+                    w[k][1] = w[k][1] + c.y;
+                }
+            u.store(t, w);
+            t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+                const T rv = r[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+                r[k][q] = rv;
+                w[k][q] = al * nb.c + be * rv;
+                if (last) t.add(acc, q, rv * rv);
+            });
+            if (last) break;
+            __syncthreads();  // every warp has read the old sd
+            ++t.tag;
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) set_operand(k, w[k][0], w[k][1]);
+            if (exchange() != RN_GO) {
+                lost = true;
+                break;
+            }
+        }
+        if (lost) break;
+        if (t.reduce(
+                acc, 1, [] {},
+                [&](double v) {
+                    s.last_beta = v / s.rro;
+                    s.rro = s.error = v;
+                    s.cheby_calc_steps = s.cheby_calc_steps + 1;
+                    end_iteration(a, s, PHASE_PPCG);
+                    return s.cont != 0;
+                },
+                [&](double v) {
+                    s.rrn = v;
+                    s.beta = s.last_beta;
+                    if (!isfinite(v)) s.nonfinite = 1;
+                }) != RN_GO)
+            break;
+    }
+    __syncthreads();  // what the last sum left to be written down
+    if (threadIdx.x == 0) {
+        s.pending_p = 1;
+        s.pending_u = 0;
+    }
+#pragma unroll
+    for (int k = 0; k < RS; ++k)
+        if (t.on(k)) {
+            const long i = t.gidx(k);
+            st_cells(a.r, i, t.both(), r[k][0], r[k][1]);
+            if constexpr (PREG) st_cells(a.p[0], i, t.both(), p[k][0], p[k][1]);
+        }
+    u.write(t);
+    RES_EPILOGUE();
+}
+
+// Jacobi: u_new = (rhs + sum K u) / diagonal and sum |u_new - u|; every 50th iteration the
+// true residual instead.
+template <class P, int RS, int W>
+__global__ void __launch_bounds__(32 * W, 1) k_res_jacobi(const __grid_constant__ ResArgs A)
+{
+    RES_PROLOGUE(P);
+    t.load_coefs(a.kx, a.ky, a.kz, nullptr);
+    t.load_operand(a.u[0]);
+    T un[RS][2];
+    const ResOwn<T, RS> b(t, a.u0);
+#pragma unroll
+    for (int k = 0; k < RS; ++k) un[k][0] = un[k][1] = (T)0;
+    __syncthreads();
+    dg.load(t);
+    for (;;) {
+        const bool residual = s.n % 50 == 0;
+        DD acc = {0.0, 0.0};
+        ++t.tag;
+        b.load(t, un);
+        t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+            const T v = jacobi_k(un[k][q], nb, kx0, kx1, ky0, ky1, kz0, kz1);
+            un[k][q] = v;
+            t.add(acc, q, fabs(v - nb.c));
+        });
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) t.publish(k, un[k][0], un[k][1]);
+        __syncthreads();  // every warp has read the old operand and the state
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) t.store(k, un[k][0], un[k][1]);
+        int next = t.reduce(
+            acc, 0, [&] { t.collect(t.nw > 1 ? 1 : 0, [&](int h, T v) { t.V[t.table()[h].x] = v; }); },
+            [&](double v) {
+                s.error = v;
+                if (!residual) end_iteration(a, s, PHASE_JACOBI);
+                return residual || s.cont != 0;
+            },
+            [](double) {});
+        if (next != RN_GO) break;
+        if (residual) {
+            acc.hi = acc.lo = 0.0;
+            b.load(t, un);
+            t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+                un[k][q] = un[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+                t.add(acc, q, un[k][q] * un[k][q]);
+            });
+#pragma unroll
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) st_cells(a.r, t.gidx(k), t.both(), un[k][0], un[k][1]);
+            next = t.reduce(
+                acc, 1, [] {},
+                [&](double v) {
+                    s.error = v;
+                    end_iteration(a, s, PHASE_JACOBI);
+                    return s.cont != 0;
+                },
+                [](double) {});
+            if (next != RN_GO) break;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < RS; ++k)
+        if (t.on(k)) {
+            const Two<T> c = ld_two(t.cell(k));
+            st_cells(a.u[0], t.gidx(k), t.both(), c.x, c.y);
+        }
+    RES_EPILOGUE();
+}
+
+}  // namespace tea

@@ -1,0 +1,80 @@
+"""The on-chip loops of the whole-solve path (one cooperative launch per loop, on grids that
+fit the SMs) against the per-call ext_* sequence, bit for bit.
+
+Sizes sit where the split can go wrong: fewer cells than a warp, one past a 64-cell strip,
+one block and many, every number of rows a warp may own, tiles cut unevenly along every axis,
+and the largest grids that fit.  The FP32 inner solves are compared with the same solve run
+one launch per sweep.  Both paths do the same operations per cell and their sums are rounded
+from twice the working precision, so nothing may differ."""
+import ctypes
+import os
+
+import numpy as np
+import pytest
+
+from conftest import same, tea
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("iterations", "error", "exact_error", "vol", "mass", "ie", "temp")
+SHAPES = {2: [(7, 5), (65, 16), (64, 17), (131, 33), (700, 37), (257, 515), (701, 699), (860, 850), (1023, 1009)],
+          3: [(5, 4, 3), (65, 9, 8), (31, 30, 29), (48, 48, 48), (66, 52, 77), (80, 77, 76)]}
+
+
+def _deck(dim, shape, solver, precond):
+    # A timestep at which the coefficients stay below about 40, so that every loop converges soon.
+    dt = 0.4 * (10.0 / max(shape)) ** 2
+    spec = tea.DeckSpec(dim=dim, cells=8, states=6, seed=sum(shape), solver=solver, end_step=2, dt=dt, eps=1e-12,
+                        max_iters=400, presteps=10, inner_steps=5 if sum(shape) % 2 else 6, preconditioner=precond,
+                        summary_frequency=1)
+    deck = tea.seeded_deck(spec)
+    for axis, n in zip("xyz", shape):
+        deck = deck.replace(f"{axis}_cells=8\n", f"{axis}_cells={n}\n")
+    return deck
+
+
+def _run(deck, dim, **kw):
+    """The run's records and its final u and energy1."""
+    lib = tea.cuda_library(dim)
+    try:
+        _, records = tea.run_deck(deck, dim, summary_every_step=True, keep_chunk=True, **kw)
+        dims = (ctypes.c_int * 3)()
+        assert lib.tea_chunk_dims_(ctypes.byref(ctypes.c_int(1)), dims) == 0
+        chunk = tea.ExtChunk.__new__(tea.ExtChunk)
+        chunk.lib, chunk.dim, chunk.id = lib, dim, 1
+        chunk.X, chunk.Y, chunk.Z = dims
+        return records, {f: chunk.read(f) for f in ("u", "energy1")}
+    finally:
+        lib.ext_finalise_()
+
+
+def _same(a, b):
+    assert len(a[0]) == len(b[0]) == 2
+    for x, y in zip(a[0], b[0]):
+        for k in FIELDS:
+            assert same(x[k], y[k]), (x["step"], k, x[k], y[k])
+    for f in a[1]:
+        assert np.array_equal(a[1][f], b[1][f], equal_nan=True), (f, np.argwhere(a[1][f] != b[1][f])[:3].tolist())
+
+
+@pytest.mark.parametrize("solver,precond", [("cg", False), ("cg", True), ("chebyshev", False), ("ppcg", False),
+                                            ("jacobi", False)])
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d]])
+def test_on_chip_loops_equal_per_call(dim, shape, solver, precond):
+    deck = _deck(dim, shape, solver, precond)
+    _same(_run(deck, dim, fused=True), _run(deck, dim))
+
+
+@pytest.mark.parametrize("solver", ["cg", "chebyshev"])
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2]])
+def test_on_chip_fp32_loops_equal_single_launches(dim, shape, solver):
+    deck = _deck(dim, shape, solver, False)
+    kw = {"fused": True, "precision": tea.PRECISION_FP32_REFINED}
+    on_chip = _run(deck, dim, **kw)
+    os.environ["TEA_B200_NO_GRAPH"] = "1"
+    try:
+        single = _run(deck, dim, **kw)
+    finally:
+        del os.environ["TEA_B200_NO_GRAPH"]
+    assert all(r["corrections"] >= 1 for r in on_chip[0])
+    _same(on_chip, single)

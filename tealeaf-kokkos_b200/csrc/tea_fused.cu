@@ -25,6 +25,7 @@
 #include "../driver/tea_eigen.h"
 #include "tea_fused.cuh"
 #include "tea_resident.cuh"
+#include "tea_stream.cuh"
 
 #define TEA_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -84,6 +85,7 @@ struct Fused {
     unsigned long long* sums = nullptr;
     unsigned long long epoch = 0;
     int sum_set = 0;
+    RingLaunch stream, stream32;  // k_stream_cg in FP64 and FP32 (blocks 0: not used)
 };
 
 // The solve state and, behind it, the failure flag of the on-chip loops, one allocation.
@@ -470,6 +472,24 @@ void res_opt_in(K kernel, size_t bytes)
     TEA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
+// Grid and work units of the streamed CG loop: one block per SM, a unit per resident warp (2D)
+// or group of warps (3D).
+template <class P>
+void setup_stream(RingLaunch& L, const Geom& g, int sms, size_t smem)
+{
+    constexpr int strip = RingGeom<typename P::T>::STRIP;
+    if (StreamRing<typename P::T>::bytes > smem) return;
+#if TEA_DIM == 2
+    const long warps = (long)sms * ST_WARPS, per_x = (g.nx + strip - 1) / strip;
+    const long per_y = std::max<long>(1, warps / per_x);
+    L.rows = (int)std::max<long>(8, (g.ny + per_y - 1) / per_y);
+#else
+    L.rows = ring3_launch(g, sms, ST_GROUPS, strip, ST_TY, sms * ST_GROUPS).rows;
+#endif
+    L.blocks = sms;
+    res_opt_in((const void*)k_stream_cg<P>, StreamRing<typename P::T>::bytes);
+}
+
 // Plans of the on-chip loops and the words their blocks exchange (rim words only for grids
 // that fit: at most 33 MB).
 void setup_resident(Chunk* c, Fused* F, int sms)
@@ -478,20 +498,23 @@ void setup_resident(Chunk* c, Fused* F, int sms)
     TEA_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     TEA_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     const size_t smem = optin > 2048 ? (size_t)optin - 2048 : 0;  // less the kernels' static part
-    if (!coop || (size_t)c->g.nx * c->g.ny * c->g.nz > (size_t)sms * RES_WARPS * 8 * 64) return;
+    sms = std::min(sms, 255);  // the arrivals at a sum are counted in a byte
+    if (!coop || c->red.max_blocks < sms) return;
+    const size_t sums = RES_SUM_WORDS * sizeof(unsigned long long);
+    TEA_CK(cudaMalloc(&F->sums, sums));
+    if (!F->sums) return;
+    TEA_CK(cudaMemsetAsync(F->sums, 0, sums, c->stream));
+    setup_stream<ResF64>(F->stream, c->g, sms, smem);
+    setup_stream<ResF32>(F->stream32, c->g, sms, smem);
+    if ((size_t)c->g.nx * c->g.ny * c->g.nz > (size_t)sms * RES_WARPS * 8 * 64) return;
     F->res[0] = res_plan(c->g, sms, sizeof(double), false, smem);
     F->res[1] = res_plan(c->g, sms, sizeof(double), true, smem);
     F->res32 = res_plan(c->g, sms, sizeof(float), false, smem);
     if (F->res[0].blocks == 0 && F->res32.blocks == 0) return;
-    const size_t rim = 2 * c->field_elems * sizeof(ResWord), sums = RES_SUM_WORDS * sizeof(unsigned long long);
+    const size_t rim = 2 * c->field_elems * sizeof(ResWord);
     TEA_CK(cudaMalloc(&F->rim, rim));
-    TEA_CK(cudaMalloc(&F->sums, sums));
-    if (!F->rim || !F->sums) {
-        F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;
-        return;
-    }
-    TEA_CK(cudaMemsetAsync(F->rim, 0, rim, c->stream));
-    TEA_CK(cudaMemsetAsync(F->sums, 0, sums, c->stream));
+    if (F->rim) TEA_CK(cudaMemsetAsync(F->rim, 0, rim, c->stream));
+    else F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;
 }
 
 template <class P, int F>
@@ -537,11 +560,9 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
     A.s0 = s;
     A.rim = F->rim;
     A.elems = (long)c->field_elems;
-    A.sums = F->sums;
-    A.set = F->sum_set;
+    A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->d_st)};
     A.scale = kind == LOOP_CHEBY || kind == LOOP_JACOBI ? s.error : s.rro;
     A.epoch = F->epoch;
-    A.fail = fail_of(F->d_st);
     const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
     res_opt_in(k, p.bytes);
     void* args[] = {&A};
@@ -553,6 +574,32 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
     }
     // More epochs than the loop can use: two rim exchanges and one per inner step an iteration.
     F->epoch += (unsigned long long)(s.max_iters + 2) * (inner_steps + 4) + 16;
+    F->sum_set ^= 1;
+    return true;
+}
+
+// Launch the CG loop of a grid that does not fit on the chip as one streaming kernel, as above.
+bool launch_stream(Chunk* c, Fused* F, int kind)
+{
+    const SolveState& s = *F->h_st;
+    if (kind != LOOP_CG && kind != LOOP_CG32) return false;
+    const bool fp32 = kind == LOOP_CG32;
+    const RingLaunch& L = fp32 ? F->stream32 : F->stream;
+    if (L.blocks == 0 || s.par_u || s.pending_p || s.pending_u) return false;
+    StreamArgs A;
+    A.f = F->base;
+    A.s0 = s;
+    A.sum = {F->sums, F->sum_set, L.blocks, fail_of(F->d_st)};
+    A.scale = s.rro;
+    A.seg = L.rows;
+    const void* k = fp32 ? (const void*)k_stream_cg<ResF32> : (const void*)k_stream_cg<ResF64>;
+    const size_t bytes = fp32 ? StreamRing<float>::bytes : StreamRing<double>::bytes;
+    void* args[] = {&A};
+    if (cudaLaunchCooperativeKernel(k, dim3(L.blocks), dim3(32 * ST_WARPS), args, bytes, c->stream) != cudaSuccess) {
+        cudaGetLastError();
+        F->stream.blocks = F->stream32.blocks = 0;
+        return false;
+    }
     F->sum_set ^= 1;
     return true;
 }
@@ -972,10 +1019,10 @@ void pull_state(Chunk* c, Fused* F)
 void run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
 {
     F->h_st->cont = 1;  // the body runs at least once (the while node's default)
-    if (launch_resident(c, F, kind, inner_steps)) {
+    if (launch_resident(c, F, kind, inner_steps) || launch_stream(c, F, kind)) {
         pull_state(c, F);
         if (*fail_of(F->h_st)) {
-            set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of an on-chip loop lost one another");
+            set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of a loop lost one another");
             TEA_CK(cudaMemsetAsync(fail_of(F->d_st), 0, sizeof(int), c->stream));
             TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
         }

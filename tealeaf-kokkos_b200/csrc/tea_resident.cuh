@@ -81,17 +81,22 @@ struct ResPlan {
     size_t bytes = 0;         // dynamic shared memory
 };
 
+struct SumArgs {
+    unsigned long long* sums;  // RES_SUM_WORDS; this launch's set is zero, the other set's words
+    int set;                   // are cleared for the next launch
+    int blocks;                // at most 255 (the arrivals are counted in a byte)
+    int* fail;
+};
+
 struct ResArgs {
     FusedArgs f;
     ResPlan p;
     SolveState s0;   // the state the loop starts from (the final one goes to *f.st)
     ResWord* rim;    // [2][elems]: rim values by the cell's array index (from the allocation's start)
     long elems;
-    unsigned long long* sums;  // RES_SUM_WORDS; this launch's set is zero, the other set's words
-    int set;                   // are cleared for the next launch
+    SumArgs sum;
     unsigned long long epoch;  // the rim exchanges' last epoch before this launch
     double scale;              // expected magnitude of the sums
-    int* fail;
 };
 
 // First cell of part i of n parts of `cells` (in units of `unit` cells).
@@ -174,6 +179,150 @@ __device__ __forceinline__ void res_limbs(double hi, double lo, int E, int (&v)[
     }
 }
 
+struct SumShared {
+    int limbs[RES_LIMBS][RES_WARPS];
+    int scale[2];  // expected exponents of the loop's two sums
+    int bad;       // a partial out of range (1) or not finite (2)
+    int next;      // what follows a sum or an iteration: RN_*
+    double sum;    // the last sum
+};
+enum { RN_GO = 0, RN_STOP = 1, RN_AGAIN = 2, RN_FAIL = 4 };
+
+// A block's part in the sums over the grid.
+struct GridSum {
+    const SumArgs& sa;
+    SumShared& ss;
+    int nw, warp, lane;
+    unsigned long long seen0 = 0, seen1 = 0;  // this lane's word of the sums, as last read, by parity
+    int parity = 0;
+    bool gave_up = false;
+
+    __device__ __forceinline__ GridSum(const SumArgs& a, SumShared& s)
+        : sa(a), ss(s), nw(blockDim.x >> 5), warp(threadIdx.x >> 5), lane(threadIdx.x & 31)
+    {
+    }
+    __device__ __forceinline__ void start(double scale)  // one thread, before the first sum
+    {
+        ss.scale[0] = ss.scale[1] = res_clamp(res_exponent(scale));
+        ss.bad = 0;
+        ss.next = RN_GO;
+    }
+    // The other set's words, by one block at the end of the launch.
+    __device__ __forceinline__ void clear_other_set() const
+    {
+        for (int i = threadIdx.x; i < RES_SUM_WORDS / 2; i += blockDim.x) sa.sums[(sa.set ^ 1) * (RES_SUM_WORDS / 2) + i] = 0;
+    }
+
+    // Sum number `which` of the loop over all blocks.  `meanwhile` runs in the other warps while
+    // warp 0 waits.  With the rounded sum, `control` runs in warp 0's first lane before any
+    // thread goes on (it returns whether the loop goes on), and `after` in the last warp's first
+    // lane while the others go on.  Returns RN_GO, RN_STOP or RN_FAIL.
+    // With FENCE, what the blocks wrote before the sum is visible to all of them after it.
+    template <bool FENCE = false, class M, class C, class N>
+    __device__ __forceinline__ int reduce(const DD& acc, int which, M&& meanwhile, C&& control, N&& after)
+    {
+        for (int tries = 0;; ++tries) {
+            const int E = ss.scale[which];
+            double hi = acc.hi, lo = acc.lo;
+            if (res_exponent(hi) > E + RES_E_ROOM) {
+                atomicOr(&ss.bad, isfinite(hi) ? 1 : 2);
+                hi = lo = 0.0;
+            }
+            int v[RES_LIMBS];
+            res_limbs(hi, lo, E, v);
+#pragma unroll
+            for (int i = 0; i < RES_LIMBS; ++i) v[i] = __reduce_add_sync(0xffffffffu, v[i]);
+            if (lane == 0) {
+#pragma unroll
+                for (int i = 0; i < RES_LIMBS; ++i) ss.limbs[i][warp] = v[i];
+            }
+            parity ^= 1;
+            __syncthreads();
+            if (warp == 0) {
+                long long mine = 0;
+#pragma unroll
+                for (int i = 0; i < RES_LIMBS; ++i) {
+                    const int w = __reduce_add_sync(0xffffffffu, lane < nw ? ss.limbs[i][lane] : 0);
+                    if (lane == i) mine = w;
+                }
+                unsigned bad = ss.bad;
+                const int nb = sa.blocks;
+                if (nb > 1) {
+                    // A count in the top byte; below it the limb, raised to be positive.  The warp
+                    // stays together: a lane that polled before another has added would wait
+                    // for a word that the other blocks' same lanes wait for too.  The atomics
+                    // return a value so that the polls begin when this block's have arrived
+                    // (1550 cycles a sum against 2050 at 64 blocks).
+                    constexpr long long bias = 1ll << 32;
+                    const bool has = lane <= RES_LIMBS;
+                    mine = lane == RES_LIMBS ? (long long)((bad & 1) + ((bad & 2) << 15)) : mine;
+                    unsigned long long* q =
+                        sa.sums + (sa.set * 2 + parity) * RES_SUM_STRIDE + (has ? lane : RES_LIMBS);
+                    const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + bias);
+                    const unsigned long long old = parity ? seen1 : seen0;
+                    unsigned long long now = old;
+                    if (FENCE) __threadfence();
+                    if (has) asm volatile("atom.relaxed.gpu.global.add.u64 %0, [%1], %2;" : "=l"(now) : "l"(q), "l"(add) : "memory");
+                    __syncwarp();
+                    now += add;
+                    for (int k = 0; __any_sync(0xffffffffu, has && (int)((now - old) >> 56) != nb); ++k) {
+                        if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)sa.fail != 0)) {
+                            gave_up = true;
+                            break;
+                        }
+                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(q) : "memory");
+                    }
+                    if (FENCE) __threadfence();
+                    mine = (long long)((now - old) & ((1ull << 56) - 1)) - nb * bias;
+                    seen0 = parity ? seen0 : now;
+                    seen1 = parity ? now : seen1;
+                    bad = (unsigned)__shfl_sync(0xffffffffu, (int)mine, RES_LIMBS);
+                    bad = ((bad & 0xffff) ? 1 : 0) | ((bad >> 16) ? 2 : 0);
+                }
+                const double part = (double)mine * res_unit(E, lane < RES_LIMBS ? lane : 0);
+                DD s = {part, 0.0};
+#pragma unroll
+                for (int i = 1; i < RES_LIMBS; ++i) dd_add(s, __shfl_sync(0xffffffffu, part, i));
+                if (lane == 0) {
+                    double sum = dd_value(s);
+                    int e = res_clamp(res_exponent(sum)), next = RN_GO;
+                    if (bad & 2) {
+                        sum = CUDART_NAN;
+                        e = E;
+                    } else if (bad) {
+                        if (E == RES_E_MAX) sum = CUDART_INF;
+                        else next = RN_AGAIN;
+                        e = min(E + 2 * RES_E_ROOM * (tries + 1), RES_E_MAX);
+                    } else if (sum == 0.0) {
+                        e = E;
+                    } else if (e < E - RES_E_LOST) {
+                        next = RN_AGAIN;
+                    }
+                    if (next == RN_GO && !control(sum)) next = RN_STOP;
+                    ss.scale[which] = e;
+                    ss.sum = sum;
+                    ss.bad = 0;
+                    ss.next = next;
+                }
+            }
+            if (tries == 0) meanwhile();
+            const int next = finish();
+            if (next & RN_FAIL) return RN_FAIL;
+            if (!(next & RN_AGAIN)) {
+                if (threadIdx.x == 32 * (nw - 1)) after(ss.sum);
+                return next;
+            }
+        }
+    }
+    // The end of an exchange: after it every thread sees what the others have written and what
+    // warp 0 has decided.
+    __device__ __forceinline__ int finish()
+    {
+        if (gave_up) *(volatile int*)sa.fail = 1;
+        return __syncthreads_or(gave_up) ? RN_FAIL : ss.next;
+    }
+};
+
 // ------------------------------------------------------------------ a block's tile
 
 template <class T>
@@ -191,15 +340,6 @@ __device__ __forceinline__ void st_two(T* p, T x, T y)
     *reinterpret_cast<Two<T>*>(p) = v;
 }
 
-struct ResShared {
-    SolveState s;
-    int limbs[RES_LIMBS][RES_WARPS];
-    int scale[2];  // expected exponents of the loop's two sums
-    int bad;       // a partial out of range (1) or not finite (2)
-    int next;      // what follows a sum or an iteration: RN_*
-    double sum;    // the last sum
-};
-enum { RN_GO = 0, RN_STOP = 1, RN_AGAIN = 2, RN_FAIL = 4 };
 
 enum {
     RF_A0 = 1, RF_A1 = 2,                // the lane's cells exist
@@ -209,14 +349,17 @@ enum {
     RF_WFIRST = 512, RF_WLAST = 1024     // the row below the first (above the last) is itself
 };
 
+struct ResShared {
+    SolveState s;
+    SumShared sum;
+};
+
 template <class T, int RS>
-struct ResTile {
+struct ResTile : GridSum {
     const ResArgs& A;
     const Geom& g;
-    ResShared& sh;
     T* const V;   // shared memory: the operand, then the arrays at the plan's offsets
     int nh;       // halo cells of this tile
-    int nw, warp, lane;
     int x0, y0, z0, tw, th, td;  // first cell (0-based inner) and extents
     int sx, plane;
     // The warp's rows: y .. y + rows - 1 of plane z, columns x and x + 1 of this lane.
@@ -226,16 +369,11 @@ struct ResTile {
     int fl;                // RF_* flags
     int dzm, dzp;          // offsets of the z-neighbours (0 at a domain face)
     unsigned long long tag;   // epoch of the last rim exchange
-    unsigned long long seen0 = 0, seen1 = 0;  // this lane's word of the sums, as last read, by parity
-    int parity = 0;
-    bool gave_up = false;
 
-    __device__ __forceinline__ ResTile(const ResArgs& a, ResShared& s, T* mem) : A(a), g(a.f.g), sh(s), V(mem)
+    __device__ __forceinline__ ResTile(const ResArgs& a, ResShared& s, T* mem)
+        : GridSum(a.sum, s.sum), A(a), g(a.f.g), V(mem)
     {
         const ResPlan& p = a.p;
-        warp = threadIdx.x >> 5;
-        lane = threadIdx.x & 31;
-        nw = blockDim.x >> 5;
         const int b = blockIdx.x;
         const int bx = b % p.nbx, by = (b / p.nbx) % p.nby, bz = b / (p.nbx * p.nby);
         x0 = res_split(g.nx, 2, bx, p.nbx);
@@ -432,114 +570,8 @@ struct ResTile {
         if (nh == 0 || warp < first) return;
         const ResWord* q = A.rim + (tag & 1) * A.elems + kLeadPad;
         for (int h = (warp - first) * 32 + lane; h < nh; h += (nw - first) * 32) {
-            put(h, res_value<T>(res_wait(q + table()[h].y, tag, A.fail, gave_up)));
+            put(h, res_value<T>(res_wait(q + table()[h].y, tag, sa.fail, gave_up)));
         }
-    }
-
-    // Sum number `which` of the loop over all blocks.  `meanwhile` runs in the other warps while
-    // warp 0 waits.  With the rounded sum, `control` runs in warp 0's first lane before any
-    // thread goes on (it returns whether the loop goes on), and `after` in the last warp's first
-    // lane while the others go on.  Returns RN_GO, RN_STOP or RN_FAIL.
-    template <class M, class C, class N>
-    __device__ __forceinline__ int reduce(const DD& acc, int which, M&& meanwhile, C&& control, N&& after)
-    {
-        for (int tries = 0;; ++tries) {
-            const int E = sh.scale[which];
-            double hi = acc.hi, lo = acc.lo;
-            if (res_exponent(hi) > E + RES_E_ROOM) {
-                atomicOr(&sh.bad, isfinite(hi) ? 1 : 2);
-                hi = lo = 0.0;
-            }
-            int v[RES_LIMBS];
-            res_limbs(hi, lo, E, v);
-#pragma unroll
-            for (int i = 0; i < RES_LIMBS; ++i) v[i] = __reduce_add_sync(0xffffffffu, v[i]);
-            if (lane == 0) {
-#pragma unroll
-                for (int i = 0; i < RES_LIMBS; ++i) sh.limbs[i][warp] = v[i];
-            }
-            parity ^= 1;
-            __syncthreads();
-            if (warp == 0) {
-                long long mine = 0;
-#pragma unroll
-                for (int i = 0; i < RES_LIMBS; ++i) {
-                    const int w = __reduce_add_sync(0xffffffffu, lane < nw ? sh.limbs[i][lane] : 0);
-                    if (lane == i) mine = w;
-                }
-                unsigned bad = sh.bad;
-                const int nb = A.p.blocks;
-                if (nb > 1) {
-                    // A count in the top byte; below it the limb, raised to be positive.  The warp
-                    // stays together: a lane that polled before another has added would wait
-                    // for a word that the other blocks' same lanes wait for too.  The atomics
-                    // return a value so that the polls begin when this block's have arrived
-                    // (1550 cycles a sum against 2050 at 64 blocks).
-                    constexpr long long bias = 1ll << 32;
-                    const bool has = lane <= RES_LIMBS;
-                    mine = lane == RES_LIMBS ? (long long)((bad & 1) + ((bad & 2) << 15)) : mine;
-                    unsigned long long* q =
-                        A.sums + (A.set * 2 + parity) * RES_SUM_STRIDE + (has ? lane : RES_LIMBS);
-                    const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + bias);
-                    const unsigned long long old = parity ? seen1 : seen0;
-                    unsigned long long now = old;
-                    if (has) asm volatile("atom.relaxed.gpu.global.add.u64 %0, [%1], %2;" : "=l"(now) : "l"(q), "l"(add) : "memory");
-                    __syncwarp();
-                    now += add;
-                    for (int k = 0; __any_sync(0xffffffffu, has && (int)((now - old) >> 56) != nb); ++k) {
-                        if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)A.fail != 0)) {
-                            gave_up = true;
-                            break;
-                        }
-                        asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(q) : "memory");
-                    }
-                    mine = (long long)((now - old) & ((1ull << 56) - 1)) - nb * bias;
-                    seen0 = parity ? seen0 : now;
-                    seen1 = parity ? now : seen1;
-                    bad = (unsigned)__shfl_sync(0xffffffffu, (int)mine, RES_LIMBS);
-                    bad = ((bad & 0xffff) ? 1 : 0) | ((bad >> 16) ? 2 : 0);
-                }
-                const double part = (double)mine * res_unit(E, lane < RES_LIMBS ? lane : 0);
-                DD s = {part, 0.0};
-#pragma unroll
-                for (int i = 1; i < RES_LIMBS; ++i) dd_add(s, __shfl_sync(0xffffffffu, part, i));
-                if (lane == 0) {
-                    double sum = dd_value(s);
-                    int e = res_clamp(res_exponent(sum)), next = RN_GO;
-                    if (bad & 2) {
-                        sum = CUDART_NAN;
-                        e = E;
-                    } else if (bad) {
-                        if (E == RES_E_MAX) sum = CUDART_INF;
-                        else next = RN_AGAIN;
-                        e = min(E + 2 * RES_E_ROOM * (tries + 1), RES_E_MAX);
-                    } else if (sum == 0.0) {
-                        e = E;
-                    } else if (e < E - RES_E_LOST) {
-                        next = RN_AGAIN;
-                    }
-                    if (next == RN_GO && !control(sum)) next = RN_STOP;
-                    sh.scale[which] = e;
-                    sh.sum = sum;
-                    sh.bad = 0;
-                    sh.next = next;
-                }
-            }
-            if (tries == 0) meanwhile();
-            const int next = finish();
-            if (next & RN_FAIL) return RN_FAIL;
-            if (!(next & RN_AGAIN)) {
-                if (threadIdx.x == 32 * (nw - 1)) after(sh.sum);
-                return next;
-            }
-        }
-    }
-    // The end of an exchange: after it every thread sees what the others have written and what
-    // warp 0 has decided.
-    __device__ __forceinline__ int finish()
-    {
-        if (gave_up) *(volatile int*)A.fail = 1;
-        return __syncthreads_or(gave_up) ? RN_FAIL : sh.next;
     }
 };
 
@@ -704,6 +736,51 @@ struct ResDiag {
     }
 };
 
+// The scalars of a CG iteration after its sums, on the block's copy of the state: alpha after
+// p.w; beta, the residual and the loop test after r.(r|z).  cg_note_* writes down what no
+// thread waits for.
+__device__ __forceinline__ bool cg_after_pw(SolveState& s, double v)
+{
+    s.alpha = s.rro / v;
+    return true;
+}
+template <class P>
+__device__ __forceinline__ void cg_note_pw(const FusedArgs& a, SolveState& s, double v)
+{
+    s.pw = v;
+    if (!P::fp32 && blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
+    if (!isfinite(v)) s.nonfinite = 1;
+}
+template <class P>
+__device__ __forceinline__ bool cg_after_rr(const FusedArgs& a, SolveState& s, double v)
+{
+    s.last_beta = v / s.rro;
+    s.rro = v;
+    if constexpr (P::fp32) {
+        const int n = ++s.n_inner;
+        const bool at_switch = s.switch_err > 0.0 && n >= s.switch_min && v <= s.switch_err;
+        s.cont = isfinite(v) && v >= s.tol2 && n < s.inner_max && !at_switch;
+    } else {
+        s.error = v;
+        end_iteration(a, s, PHASE_CG);
+    }
+    return s.cont != 0;
+}
+template <class P>
+__device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, double v)
+{
+    // The iteration that has just ended: end_iteration steps n unless it converged.
+    const int n = P::fp32 ? s.n_inner : (s.exit_reason == EXIT_CONVERGED ? s.n : s.n - 1);
+    s.rrn = v;
+    s.beta = s.last_beta;
+    s.last_alpha = s.alpha;
+    if (!isfinite(v)) s.nonfinite = 1;
+    if (blockIdx.x == 0) {
+        if (P::fp32) a.cg_alphas[n] = s.alpha;
+        a.cg_betas[n] = s.beta;
+    }
+}
+
 #define RES_PROLOGUE(P)                                                                            \
     using T = typename P::T;                                                                       \
     extern __shared__ __align__(16) unsigned char s_res_raw[];                                     \
@@ -711,11 +788,9 @@ struct ResDiag {
     const FusedArgs& a = A.f;                                                                      \
     if (threadIdx.x == 0) {                                                                        \
         sh.s = A.s0;                                                                               \
-        sh.scale[0] = sh.scale[1] = res_clamp(res_exponent(A.scale));                              \
-        sh.bad = 0;                                                                                \
-        sh.next = RN_GO;                                                                           \
     }                                                                                              \
     ResTile<T, RS> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                      \
+    if (threadIdx.x == 0) t.start(A.scale);                                                        \
     ResDiag<T, RS> dg;                                                                             \
     SolveState& s = sh.s
 
@@ -723,8 +798,7 @@ struct ResDiag {
     __syncthreads();                                                                               \
     if (blockIdx.x == 0) {                                                                         \
         if (threadIdx.x == 0) *a.st = s;                                                           \
-        for (int i = threadIdx.x; i < RES_SUM_WORDS / 2; i += blockDim.x)                          \
-            A.sums[(A.set ^ 1) * (RES_SUM_WORDS / 2) + i] = 0;                                     \
+        t.clear_other_set();                                                                       \
     }
 
 // CG: per iteration p = beta p + (z|r), w = A p and p.w; u += alpha p, r -= alpha w and
@@ -777,16 +851,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
             t.add(acc, q, (double)wv * (double)nb.c);
         });
         if (t.reduce(
-                acc, 0, [] {},
-                [&](double v) {
-                    s.alpha = s.rro / v;
-                    return true;
-                },
-                [&](double v) {
-                    s.pw = v;
-                    if (!P::fp32 && blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
-                    if (!isfinite(v)) s.nonfinite = 1;
-                }) != RN_GO)
+                acc, 0, [] {}, [&](double v) { return cg_after_pw(s, v); }, [&](double v) { cg_note_pw<P>(a, s, v); }) !=
+            RN_GO)
             break;
         const T alpha = (T)s.alpha;
         acc.hi = acc.lo = 0.0;
@@ -816,34 +882,10 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
                 w[k][1] = w[k][1] + alpha * c.y;
             }
         u.store(t, w);
-        const int next = t.reduce(
-            acc, 1, [&] { t.collect(1, [&](int h, T v) { t.halo_r(h) = v; }); },
-            [&](double v) {
-                s.last_beta = v / s.rro;
-                s.rro = v;
-                if constexpr (P::fp32) {
-                    const int n = ++s.n_inner;
-                    const bool at_switch = s.switch_err > 0.0 && n >= s.switch_min && v <= s.switch_err;
-                    s.cont = isfinite(v) && v >= s.tol2 && n < s.inner_max && !at_switch;
-                } else {
-                    s.error = v;
-                    end_iteration(a, s, PHASE_CG);
-                }
-                return s.cont != 0;
-            },
-            [&](double v) {
-                // The iteration that has just ended: end_iteration steps n unless it converged.
-                const int n = P::fp32 ? s.n_inner : (s.exit_reason == EXIT_CONVERGED ? s.n : s.n - 1);
-                s.rrn = v;
-                s.beta = s.last_beta;
-                s.last_alpha = s.alpha;
-                if (!isfinite(v)) s.nonfinite = 1;
-                if (blockIdx.x == 0) {
-                    if (P::fp32) a.cg_alphas[n] = s.alpha;
-                    a.cg_betas[n] = s.beta;
-                }
-            });
-        if (next != RN_GO) break;
+        if (t.reduce(
+                acc, 1, [&] { t.collect(1, [&](int h, T v) { t.halo_r(h) = v; }); },
+                [&](double v) { return cg_after_rr<P>(a, s, v); }, [&](double v) { cg_note_rr<P>(a, s, v); }) != RN_GO)
+            break;
     }
     __syncthreads();  // what the last sum left to be written down
     t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
@@ -928,7 +970,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
         if (check) {
             next = t.reduce(acc, 0, [&] { halo(t.nw > 1 ? 1 : 0); }, finish, [](double) {});
         } else {
-            if (threadIdx.x == 0) sh.next = finish(0.0) ? RN_GO : RN_STOP;
+            if (threadIdx.x == 0) sh.sum.next = finish(0.0) ? RN_GO : RN_STOP;
             halo(0);
             next = t.finish();
         }

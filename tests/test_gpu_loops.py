@@ -1,5 +1,5 @@
-"""The on-chip loops of the whole-solve path (one cooperative launch per loop, on grids that
-fit the SMs) against the per-call ext_* sequence, bit for bit.
+"""The one-launch loops of the whole-solve path against the per-call ext_* sequence, bit for bit:
+the on-chip loops of grids that fit the SMs and the streaming CG loop of those that do not.
 
 Sizes sit where the split can go wrong: fewer cells than a warp, one past a 64-cell strip,
 one block and many, every number of rows a warp may own, tiles cut unevenly along every axis,
@@ -17,6 +17,8 @@ from conftest import same, tea
 pytestmark = pytest.mark.gpu
 
 FIELDS = ("iterations", "error", "exact_error", "vol", "mass", "ie", "temp")
+# Too large for the chip: the streaming CG loop, on ragged sides and on few and many work units.
+STREAM_SHAPES = {2: [(1101, 1003), (4099, 300), (300, 4100)], 3: [(101, 99, 97), (3, 200, 100), (257, 66, 65)]}
 SHAPES = {2: [(7, 5), (65, 16), (64, 17), (131, 33), (700, 37), (257, 515), (701, 699), (860, 850), (1023, 1009)],
           3: [(5, 4, 3), (65, 9, 8), (31, 30, 29), (48, 48, 48), (66, 52, 77), (80, 77, 76)]}
 
@@ -65,9 +67,16 @@ def test_on_chip_loops_equal_per_call(dim, shape, solver, precond):
     _same(_run(deck, dim, fused=True), _run(deck, dim))
 
 
+@pytest.mark.parametrize("precond", [False, True])
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in STREAM_SHAPES[d]])
+def test_streaming_cg_equals_per_call(dim, shape, precond):
+    deck = _deck(dim, shape, "cg", precond)
+    _same(_run(deck, dim, fused=True), _run(deck, dim))
+
+
 @pytest.mark.parametrize("solver", ["cg", "chebyshev"])
-@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2]])
-def test_on_chip_fp32_loops_equal_single_launches(dim, shape, solver):
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2] + STREAM_SHAPES[d][::2]])
+def test_one_launch_fp32_loops_equal_single_launches(dim, shape, solver):
     deck = _deck(dim, shape, solver, False)
     kw = {"fused": True, "precision": tea.PRECISION_FP32_REFINED}
     on_chip = _run(deck, dim, **kw)

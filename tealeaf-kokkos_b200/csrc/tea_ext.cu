@@ -303,12 +303,19 @@ void update_halo(Chunk* c, const int* neighbours, const int* fields, int depth)
         set_status(2, "ext_update_halo_kernel_: depth %d outside 1..%d", depth, HALO_PAD);
         return;
     }
-    // Two phases in 2D (left/right span the halo rows that top/bottom then copy); one in 3D.
-    const int nphase = DIM == 2 ? 2 : 1;
+    // In 2D the left and right faces span the halo rows, which the bottom and top faces then copy:
+    // one launch that works the corners out itself when both sides of an axis have their own
+    // cells to mirror, else two.  One launch in 3D.
+    const bool at_once = DIM == 3 || (g.nx >= 2 && g.ny >= 2);
+    const int nphase = at_once ? 1 : 2;
     for (int phase = 0; phase < nphase; ++phase) {
         HaloJob job;
         job.nseg = 0;
         job.depth = depth;
+        job.sides = 0;
+        if (DIM == 2 && at_once)
+            for (int face = 1; face <= 4; ++face)
+                if (neighbours[face - 1] == -1) job.sides |= 1 << (face - 1);
         long maxcount = 0;
         for (int fid = 1; fid <= 6; ++fid) {
             if (!fields[fid - 1]) continue;
@@ -319,7 +326,7 @@ void update_halo(Chunk* c, const int* neighbours, const int* fields, int depth)
                 long count;
                 if (DIM == 2) {
                     const bool lr = face <= 2;
-                    if ((phase == 0) != lr) continue;
+                    if (!at_once && (phase == 0) != lr) continue;
                     count = lr ? (long)g.Y * depth : (long)g.X * depth;
                 } else {
                     if (face <= 2) count = (long)g.ny * g.nz * depth;

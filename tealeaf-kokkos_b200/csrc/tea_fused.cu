@@ -26,6 +26,7 @@
 #include "tea_fused.cuh"
 #include "tea_resident.cuh"
 #include "tea_stream.cuh"
+#include "tea_ends.cuh"
 
 #define TEA_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -56,7 +57,10 @@ constexpr int RING_OPS = 9;
 
 struct Fused {
     SolveState* d_st = nullptr;
-    SolveState* h_st = nullptr;  // pinned
+    SolveState* d_start = nullptr;  // the state a set-up leaves for the first loop
+    SolveState* h_st = nullptr;     // pinned and mapped; behind it the loops' failure flag
+    SolveState* m_st = nullptr;     // its device alias
+    double* h_coefs = nullptr;      // pinned staging of the CG scalars and the Chebyshev coefficients
     double* alt[3] = {nullptr, nullptr, nullptr};  // allocations of u, p, sd second buffers
     float* alloc32[10] = {};  // FP32 arrays of the defect-correction form (allocated on first use)
     double *d_cg_alphas = nullptr, *d_cg_betas = nullptr;
@@ -88,7 +92,7 @@ struct Fused {
     RingLaunch stream, stream32;  // k_stream_cg in FP64 and FP32 (blocks 0: not used)
 };
 
-// The solve state and, behind it, the failure flag of the on-chip loops, one allocation.
+// The host's solve state and, behind it, the failure flag of the one-launch loops.
 constexpr size_t kStateBytes = (sizeof(SolveState) + 15) / 16 * 16 + 16;
 inline int* fail_of(SolveState* s)
 {
@@ -545,9 +549,10 @@ const void* res_kernel(int kind, int form)
     }
 }
 
-// Launch loop `kind` as one on-chip kernel from the host's state; false when the grid, the loop
-// or the state is not of a form it takes (then the loop runs as a graph).
-bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
+// Launch loop `kind` as one on-chip kernel from the host's state or, with `started`, from the state
+// that the set-up leaves in d_start (the host's has the same flags); false when the grid, the
+// loop or the state is not of a form it takes (then the loop runs as a graph).
+bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started)
 {
     const SolveState& s = *F->h_st;
     const bool fp32 = kind == LOOP_CG32 || kind == LOOP_CHEBY32;
@@ -557,11 +562,12 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
     ResArgs A;
     A.f = F->base;
     A.p = p;
+    A.start = started ? F->d_start : nullptr;
     A.s0 = s;
+    A.host = F->m_st;
     A.rim = F->rim;
     A.elems = (long)c->field_elems;
-    A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->d_st)};
-    A.scale = kind == LOOP_CHEBY || kind == LOOP_JACOBI ? s.error : s.rro;
+    A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->m_st)};
     A.epoch = F->epoch;
     const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
     res_opt_in(k, p.bytes);
@@ -579,7 +585,7 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps)
 }
 
 // Launch the CG loop of a grid that does not fit on the chip as one streaming kernel, as above.
-bool launch_stream(Chunk* c, Fused* F, int kind)
+bool launch_stream(Chunk* c, Fused* F, int kind, bool started)
 {
     const SolveState& s = *F->h_st;
     if (kind != LOOP_CG && kind != LOOP_CG32) return false;
@@ -588,9 +594,10 @@ bool launch_stream(Chunk* c, Fused* F, int kind)
     if (L.blocks == 0 || s.par_u || s.pending_p || s.pending_u) return false;
     StreamArgs A;
     A.f = F->base;
+    A.start = started ? F->d_start : nullptr;
     A.s0 = s;
-    A.sum = {F->sums, F->sum_set, L.blocks, fail_of(F->d_st)};
-    A.scale = s.rro;
+    A.host = F->m_st;
+    A.sum = {F->sums, F->sum_set, L.blocks, fail_of(F->m_st)};
     A.seg = L.rows;
     const void* k = fp32 ? (const void*)k_stream_cg<ResF32> : (const void*)k_stream_cg<ResF64>;
     const size_t bytes = fp32 ? StreamRing<float>::bytes : StreamRing<double>::bytes;
@@ -612,9 +619,12 @@ Fused* ensure_fused(Chunk* c, int max_iters)
         c->fused = F;
         const char* env = std::getenv("TEA_B200_NO_GRAPH");
         F->use_graph = !(env && env[0] == '1');
-        TEA_CK(cudaMalloc(&F->d_st, kStateBytes));
-        TEA_CK(cudaMemset(F->d_st, 0, kStateBytes));
-        TEA_CK(cudaHostAlloc(&F->h_st, kStateBytes, cudaHostAllocDefault));
+        TEA_CK(cudaMalloc(&F->d_st, 2 * sizeof(SolveState)));
+        TEA_CK(cudaMemset(F->d_st, 0, 2 * sizeof(SolveState)));
+        F->d_start = F->d_st + 1;
+        TEA_CK(cudaHostAlloc(&F->h_st, kStateBytes, cudaHostAllocMapped));
+        std::memset((void*)F->h_st, 0, kStateBytes);
+        TEA_CK(cudaHostGetDevicePointer(&F->m_st, F->h_st, 0));
         for (int k = 0; k < 3; ++k) {
             TEA_CK(cudaMalloc(&F->alt[k], c->field_elems * sizeof(double)));
             if (F->alt[k]) TEA_CK(cudaMemset(F->alt[k], 0, c->field_elems * sizeof(double)));
@@ -760,6 +770,8 @@ Fused* ensure_fused(Chunk* c, int max_iters)
         for (double* p : {F->d_cg_alphas, F->d_cg_betas, F->d_ch_alphas, F->d_ch_betas})
             if (p) TEA_CK(cudaFree(p));
         F->cap = max_iters + 2;
+        if (F->h_coefs) TEA_CK(cudaFreeHost(F->h_coefs));
+        TEA_CK(cudaHostAlloc(&F->h_coefs, 2 * sizeof(double) * F->cap, cudaHostAllocDefault));
         TEA_CK(cudaMalloc(&F->d_cg_alphas, sizeof(double) * F->cap));
         TEA_CK(cudaMalloc(&F->d_cg_betas, sizeof(double) * F->cap));
         TEA_CK(cudaMalloc(&F->d_ch_alphas, sizeof(double) * F->cap));
@@ -1010,22 +1022,34 @@ void push_state(Chunk* c, Fused* F)
 
 void pull_state(Chunk* c, Fused* F)
 {
-    TEA_CK(cudaMemcpyAsync(F->h_st, F->d_st, kStateBytes, cudaMemcpyDeviceToHost, c->stream));
-    c->d2h_bytes += kStateBytes;
+    TEA_CK(cudaMemcpyAsync(F->h_st, F->d_st, sizeof(SolveState), cudaMemcpyDeviceToHost, c->stream));
+    c->d2h_bytes += sizeof(SolveState);
     sync(c);
+}
+
+bool launch_loop(Chunk* c, Fused* F, int kind, int inner_steps, bool started)
+{
+    return launch_resident(c, F, kind, inner_steps, started) || launch_stream(c, F, kind, started);
+}
+
+// Waits for a loop launched by launch_loop, which has left its final state in the host's record.
+void await_loop(Chunk* c, Fused* F)
+{
+    sync(c);
+    c->d2h_bytes += sizeof(SolveState);
+    if (*(volatile int*)fail_of(F->h_st)) {
+        set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of a loop lost one another");
+        *fail_of(F->h_st) = 0;
+        TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
+    }
 }
 
 // Run loop `kind` from the current state until its exit; the host state is refreshed.
 void run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
 {
     F->h_st->cont = 1;  // the body runs at least once (the while node's default)
-    if (launch_resident(c, F, kind, inner_steps) || launch_stream(c, F, kind)) {
-        pull_state(c, F);
-        if (*fail_of(F->h_st)) {
-            set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of a loop lost one another");
-            TEA_CK(cudaMemsetAsync(fail_of(F->d_st), 0, sizeof(int), c->stream));
-            TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
-        }
+    if (launch_loop(c, F, kind, inner_steps, false)) {
+        await_loop(c, F);
         return;
     }
     push_state(c, F);
@@ -1082,32 +1106,40 @@ void halo(Chunk* c, std::initializer_list<int> ids, int depth)
     update_halo(c, kAllExternal, fields, depth);
 }
 
-// Bring u and p to the state the per-call kernels expect: pending updates applied,
-// current values in the canonical buffers, the depth-1 halo of u reflected and that of
-// p reflected when the reference's halo field list holds p at this point (it does not
-// in Chebyshev mode before a CG iteration has run, tealeaf_2d/tea_solve.f90:203-204).
-void canonicalize(Chunk* c, Fused* F, bool refresh_p = true)
+// Bring u and p to the state the per-call kernels expect (k_settle).  The halo of p is reflected
+// when the reference's halo field list holds p at this point (it does not in Chebyshev mode
+// before a CG iteration has run, tealeaf_2d/tea_solve.f90:203-204).
+void canonicalize(Chunk* c, Fused* F, bool refresh_p = true, bool energy = false)
 {
     SolveState& s = *F->h_st;
-    FusedArgs a = F->base;
-    if (s.pending_p || s.pending_u) {
-        push_state(c, F);
-        k_flush<<<F->point_blocks, dim3(TILE_X, TILE_Y), 0, c->stream>>>(a, c->inner);
-        s.pending_p = 0;
-        s.pending_u = 0;
-    }
-    const size_t bytes = c->field_elems * sizeof(double);
-    if (s.par_p) {
-        TEA_CK(cudaMemcpyAsync(c->alloc[F_P], F->alt[1], bytes, cudaMemcpyDeviceToDevice, c->stream));
-        s.par_p = 0;
-    }
-    if (s.par_u) {
-        TEA_CK(cudaMemcpyAsync(c->alloc[F_U], F->alt[0], bytes, cudaMemcpyDeviceToDevice, c->stream));
-        s.par_u = 0;
-    }
-    push_state(c, F);
-    if (refresh_p) halo(c, {4, 5}, 1);
-    else halo(c, {4}, 1);
+    k_settle<<<F->point_blocks, dim3(TILE_X, TILE_Y), 0, c->stream>>>(F->base, c->f, c->inner, s, nullptr,
+                                                                     refresh_p ? 1 : 0, energy ? 1 : 0);
+    TEA_CK(cudaGetLastError());
+    s.pending_p = s.pending_u = 0;
+    s.par_p = s.par_u = 0;
+}
+
+// The set-up of a CG, Chebyshev or PPCG solve in one launch; `s` is the starting state but for
+// rro and a relative eps.  Nothing waits for it.
+void launch_setup(Chunk* c, Fused* F, const tea_solve_params* P, const SolveState& s)
+{
+    c->preconditioner = s.precond;
+    SetupArgs a;
+    a.g = c->g;
+    a.f = c->f;
+    a.full = c->full;
+    a.cond = P->coefficient == 1 ? 1 : 0;
+    a.precond = s.precond;
+    a.rx = P->dt / (c->dx * c->dx);
+    a.ry = P->dt / (c->dy * c->dy);
+    a.rz = DIM == 3 ? P->dt / (c->dz * c->dz) : 0.0;
+    a.eps_rel = P->eps_rel;
+    a.red = c->red;
+    a.s0 = s;
+    a.start = F->d_start;
+    a.out = c->d_out;
+    k_setup<<<launch_blocks(c, c->full.ntiles), dim3(TILE_X, TILE_Y), 0, c->stream>>>(a);
+    TEA_CK(cudaGetLastError());
 }
 
 }  // namespace
@@ -1127,6 +1159,7 @@ void destroy_fused(Chunk* c)
     if (F->sums) cudaFree(F->sums);
     if (F->d_st) cudaFree(F->d_st);
     if (F->h_st) cudaFreeHost(F->h_st);
+    if (F->h_coefs) cudaFreeHost(F->h_coefs);
     delete F;
     c->fused = nullptr;
 }
@@ -1153,22 +1186,56 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
     int coefficient = P->coefficient, precond = P->preconditioner ? 1 : 0;
     double dt = P->dt;
 
-    // INIT, tealeaf_2d/tea_solve.f90:79-164.
-    halo(c, {3, 1}, 2);
-    double rro = 0.0;
-    if (cg_like) {
-        ext_cg_solver_init_(chunk, &coefficient, &precond, &dt, &rro);
-        halo(c, {4, 5}, 1);
+    SolveState& s = *F->h_st;
+    std::memset((void*)&s, 0, sizeof(s));
+    s.error = 1e10;
+    s.eps = P->eps;
+    s.epslim = P->ch_cg_epslim;
+    s.n = 1;
+    s.cont = 1;
+    s.solver = solver;
+    s.precond = precond;
+    s.max_iters = P->max_iters;
+    s.presteps = P->ch_cg_presteps;
+    s.errswitch = P->ch_cg_errswitch ? 1 : 0;
+    s.inner_steps = P->ppcg_inner_steps;
+
+    // INIT, tealeaf_2d/tea_solve.f90:79-164: one launch; the first CG loop of a plain solve, and
+    // the end of a CG solve, follow it without a word from the host.  Jacobi, and grids one cell
+    // wide along an axis (whose halo mirrors itself), are set up by the per-call kernels.
+    double rro = 0.0, eps = P->eps;
+    bool running = false, settled = false;
+    if (cg_like && coefficient >= 1 && c->g.nx > 1 && c->g.ny > 1 && (DIM == 2 || c->g.nz > 1)) {
+        launch_setup(c, F, P, s);
+        running = !c->ws && P->precision == TEA_PRECISION_FP64 && launch_loop(c, F, LOOP_CG, 0, true);
+        if (running && solver == TEA_SOLVER_CG) {
+            k_settle<<<F->point_blocks, dim3(TILE_X, TILE_Y), 0, c->stream>>>(F->base, c->f, c->inner, s, F->d_st, 1, 1);
+            settled = true;
+        }
+        if (running) {
+            await_loop(c, F);
+            eps = s.eps;
+        } else {
+            sync(c);
+            rro = ((volatile double*)c->h_out)[0];
+            if (P->eps_rel > 0.0) eps = P->eps_rel * P->eps_rel * ((volatile double*)c->h_out)[1];
+            c->d2h_bytes += 2 * sizeof(double);
+        }
     } else {
-        ext_jacobi_kernel_init_(chunk, &coefficient, &dt);
-    }
-    ext_solver_copy_u_(chunk);
-    double eps = P->eps;
-    if (P->eps_rel > 0.0) {
-        double bb = 0.0;
-        int zero = 0;
-        ext_calculate_2norm_(chunk, &bb, &zero);
-        eps = P->eps_rel * P->eps_rel * bb;
+        halo(c, {3, 1}, 2);
+        if (cg_like) {
+            ext_cg_solver_init_(chunk, &coefficient, &precond, &dt, &rro);
+            halo(c, {4, 5}, 1);
+        } else {
+            ext_jacobi_kernel_init_(chunk, &coefficient, &dt);
+        }
+        ext_solver_copy_u_(chunk);
+        if (P->eps_rel > 0.0) {
+            double bb = 0.0;
+            int zero = 0;
+            ext_calculate_2norm_(chunk, &bb, &zero);
+            eps = P->eps_rel * P->eps_rel * bb;
+        }
     }
     // Learned warm start (a network attached with tea_ws_attach_): keep u = u0 + du when its
     // FP64 residual is smaller than that of u = u0, and restart CG from it.  After three
@@ -1206,25 +1273,10 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
             }
         }
     }
-    // The second buffers start as copies, so halos the loops never write match u and p.
-    const size_t bytes = c->field_elems * sizeof(double);
-    TEA_CK(cudaMemcpyAsync(F->alt[0], c->alloc[F_U], bytes, cudaMemcpyDeviceToDevice, c->stream));
-    TEA_CK(cudaMemcpyAsync(F->alt[1], c->alloc[F_P], bytes, cudaMemcpyDeviceToDevice, c->stream));
-
-    SolveState& s = *F->h_st;
-    std::memset(&s, 0, sizeof(s));
-    s.rro = rro;
-    s.error = 1e10;
-    s.eps = eps;
-    s.epslim = P->ch_cg_epslim;
-    s.n = 1;
-    s.cont = 1;
-    s.solver = solver;
-    s.precond = precond;
-    s.max_iters = P->max_iters;
-    s.presteps = P->ch_cg_presteps;
-    s.errswitch = P->ch_cg_errswitch ? 1 : 0;
-    s.inner_steps = P->ppcg_inner_steps;
+    if (!running) {
+        s.rro = rro;
+        s.eps = eps;
+    }
     const bool cheby = solver == TEA_SOLVER_CHEBYSHEV, ppcg = solver == TEA_SOLVER_PPCG;
     int switch_step = 0, cg_steps = 0;
     double eigmin = 0.0, eigmax = 0.0;
@@ -1360,16 +1412,16 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                     // The switch, tealeaf_2d/tea_solve.f90:184-223, on the host.
                     canonicalize(c, F);
                     cg_steps = n - 1;
-                    std::vector<double> ca(n + 1, 0.0), cb(n + 1, 0.0);
-                    TEA_CK(cudaMemcpyAsync(ca.data(), F->d_cg_alphas, sizeof(double) * (n + 1),
-                                           cudaMemcpyDeviceToHost, c->stream));
-                    TEA_CK(cudaMemcpyAsync(cb.data(), F->d_cg_betas, sizeof(double) * (n + 1),
-                                           cudaMemcpyDeviceToHost, c->stream));
+                    double *ca = F->h_coefs, *cb = F->h_coefs + F->cap;
+                    TEA_CK(cudaMemcpyAsync(ca, F->d_cg_alphas, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost,
+                                           c->stream));
+                    TEA_CK(cudaMemcpyAsync(cb, F->d_cg_betas, sizeof(double) * (n + 1), cudaMemcpyDeviceToHost,
+                                           c->stream));
                     sync(c);
                     c->d2h_bytes += 2 * sizeof(double) * (long long)(n + 1);
                     max_cheby_iters = P->max_iters - n + 2;
                     s.rro = s.error;
-                    int info = tea_calc_eigenvalues(ca.data() + 1, cb.data() + 1, n - 1, &eigmin, &eigmax);
+                    int info = tea_calc_eigenvalues(ca + 1, cb + 1, n - 1, &eigmin, &eigmax);
                     if (info != 0) {
                         set_status(TEA_ERR_EIGEN, "tea_leaf: Error in calculating eigenvalues");
                         R->status = TEA_ERR_EIGEN;
@@ -1384,10 +1436,10 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                                       cheby ? max_cheby_iters : P->ppcg_inner_steps);
                     cn = eigmax / eigmin;
                     const int nup = std::min<int>((int)ch_alphas.size(), F->cap);
-                    TEA_CK(cudaMemcpyAsync(F->d_ch_alphas, ch_alphas.data(), sizeof(double) * nup,
-                                           cudaMemcpyHostToDevice, c->stream));
-                    TEA_CK(cudaMemcpyAsync(F->d_ch_betas, ch_betas.data(), sizeof(double) * nup,
-                                           cudaMemcpyHostToDevice, c->stream));
+                    std::copy(ch_alphas.begin(), ch_alphas.begin() + nup, ca);
+                    std::copy(ch_betas.begin(), ch_betas.begin() + nup, cb);
+                    TEA_CK(cudaMemcpyAsync(F->d_ch_alphas, ca, sizeof(double) * nup, cudaMemcpyHostToDevice, c->stream));
+                    TEA_CK(cudaMemcpyAsync(F->d_ch_betas, cb, sizeof(double) * nup, cudaMemcpyHostToDevice, c->stream));
                     c->h2d_bytes += 2 * sizeof(double) * (long long)nup;
                     switch_step = n;
                     if (cheby) {
@@ -1432,16 +1484,8 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                         halo(c, {4, 5}, 1);
                         end_iteration_host(s, PHASE_PPCG);
                     }
-                    // Fresh copies for the second buffers (halos as in the canonical ones).
-                    TEA_CK(cudaMemcpyAsync(F->alt[0], c->alloc[F_U], bytes, cudaMemcpyDeviceToDevice, c->stream));
-                    TEA_CK(cudaMemcpyAsync(F->alt[1], c->alloc[F_P], bytes, cudaMemcpyDeviceToDevice, c->stream));
                     if (s.exit_reason == EXIT_CONVERGED || s.exit_reason == EXIT_MAXITER) break;
                     continue;
-                }
-                if (cheby) {
-                    // The Chebyshev loop may leave p in the second buffer; both start with the
-                    // same contents, so the halo (never written in this phase) agrees.
-                    TEA_CK(cudaMemcpyAsync(F->alt[1], c->alloc[F_P], bytes, cudaMemcpyDeviceToDevice, c->stream));
                 }
                 run_loop(c, F, cheby ? LOOP_CHEBY : LOOP_PPCG, P->ppcg_inner_steps);
             } else if (!p_halo_fresh) {
@@ -1462,6 +1506,8 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                 push_state(c, F);
                 if (s.exit_reason == EXIT_CONVERGED || s.exit_reason == EXIT_MAXITER) break;
                 continue;
+            } else if (running) {
+                running = false;  // the CG loop that followed the set-up
             } else {
                 run_loop(c, F, LOOP_CG, 0);
             }
@@ -1469,7 +1515,7 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
             canonicalize(c, F, p_halo_fresh);
         }
     }
-    canonicalize(c, F);
+    if (!settled) canonicalize(c, F, true, true);
     if (s.nonfinite) set_status(TEA_ERR_NONFINITE, "ext_tea_leaf_solve_: non-finite value in a reduction");
     double exact_error = 0.0;
     if (P->check_result) {
@@ -1477,8 +1523,6 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
         ext_calculate_residual_(chunk);
         ext_calculate_2norm_(chunk, &exact_error, &one);
     }
-    ext_solver_finalise_(chunk);
-    halo(c, {3}, 1);
     sync(c);
     R->iterations = s.n - 1;
     R->status = status_store().status;

@@ -3134,31 +3134,4 @@ __global__ void __launch_bounds__(256) k_dc_update(FusedArgs a)
     });
 }
 
-// ------------------------------------------------------------------ flush
-
-// Applies what the fused CG/PPCG loop left pending so that u and p hold exactly what the
-// reference's per-iteration calls would have left: u += last_alpha p, p = last_beta p +
-// (z|r), both in place on the current buffers.
-__global__ void __launch_bounds__(BLOCK) k_flush(FusedArgs a, Box inner)
-{
-    const SolveState& s = *a.st;
-    if (!s.pending_p && !s.pending_u) return;
-    double* p = a.p[s.par_p];
-    const double alpha = s.last_alpha, beta = s.last_beta;
-    const int pu = s.pending_u, pp = s.pending_p, precond = s.precond;
-    const Geom& g = a.g;
-    walk(inner, [&](int kk, int jj, int ii) {
-        const long i = fidx(g, kk, jj, ii);
-        const double po = p[i];
-        if (pu) a.u[0][i] = a.u[0][i] + alpha * po;
-        if (pp) p[i] = beta * po + (precond ? a.z[i] : a.r[i]);
-    });
-}
-
-__global__ void k_clear_pending(SolveState* s)
-{
-    s->pending_p = 0;
-    s->pending_u = 0;
-}
-
 }  // namespace tea

@@ -239,6 +239,7 @@ struct HaloJob {
     HaloSeg seg[36];
     int nseg;
     int depth;
+    int sides;  // 2D, all faces in one launch: the external faces (bit face - 1); 0: one axis a launch
 };
 
 // UpdateHalo, tealeaf_2d/ext_update_halo.hpp:12-76 (3D :12-136).  2D faces span the whole
@@ -258,12 +259,19 @@ __global__ void k_update_halo(Geom g, HaloJob job)
             const int kf = sg.face == 1 ? HALO_PAD + fl : g.X - HALO_PAD - 1 - fl;
             to = fidx(g, kt, jj, 0);
             from = fidx(g, kf, jj, 0);
+            // Halo rows that the bottom or top face writes are left to it.
+            if ((job.sides & 4) && jj < HALO_PAD && jj >= HALO_PAD - depth) continue;
+            if ((job.sides & 8) && jj >= g.Y - HALO_PAD && jj < g.Y - HALO_PAD + depth) continue;
         } else {
             const int kk = (int)(idx % g.X), fl = (int)(idx / g.X);
             const int jt = sg.face == 3 ? HALO_PAD - 1 - fl : g.Y - HALO_PAD + fl;
             const int jf = sg.face == 3 ? HALO_PAD + fl : g.Y - HALO_PAD - 1 - fl;
             to = fidx(g, kk, jt, 0);
-            from = fidx(g, kk, jf, 0);
+            // What the left or right face gives the column.
+            int kf = kk;
+            if ((job.sides & 1) && kk < HALO_PAD && kk >= HALO_PAD - depth) kf = 2 * HALO_PAD - 1 - kk;
+            if ((job.sides & 2) && kk >= g.X - HALO_PAD && kk < g.X - HALO_PAD + depth) kf = 2 * (g.X - HALO_PAD) - 1 - kk;
+            from = fidx(g, kf, jf, 0);
         }
 #else
         if (sg.face == 1 || sg.face == 2) {

@@ -91,12 +91,13 @@ struct SumArgs {
 struct ResArgs {
     FusedArgs f;
     ResPlan p;
-    SolveState s0;   // the state the loop starts from (the final one goes to *f.st)
+    const SolveState* start;  // the state the loop starts from, or null: s0
+    SolveState s0;
+    SolveState* host;  // the final state goes to *f.st and to the host's record
     ResWord* rim;    // [2][elems]: rim values by the cell's array index (from the allocation's start)
     long elems;
     SumArgs sum;
     unsigned long long epoch;  // the rim exchanges' last epoch before this launch
-    double scale;              // expected magnitude of the sums
 };
 
 // First cell of part i of n parts of `cells` (in units of `unit` cells).
@@ -781,23 +782,23 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
     }
 }
 
-#define RES_PROLOGUE(P)                                                                            \
+#define RES_PROLOGUE(P, RES_SCALE)                                                                 \
     using T = typename P::T;                                                                       \
     extern __shared__ __align__(16) unsigned char s_res_raw[];                                     \
     __shared__ ResShared sh;                                                                       \
     const FusedArgs& a = A.f;                                                                      \
     if (threadIdx.x == 0) {                                                                        \
-        sh.s = A.s0;                                                                               \
+        sh.s = A.start ? *A.start : A.s0;                                                          \
     }                                                                                              \
     ResTile<T, RS> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                      \
-    if (threadIdx.x == 0) t.start(A.scale);                                                        \
+    if (threadIdx.x == 0) t.start(RES_SCALE);                                                      \
     ResDiag<T, RS> dg;                                                                             \
     SolveState& s = sh.s
 
 #define RES_EPILOGUE()                                                                             \
     __syncthreads();                                                                               \
     if (blockIdx.x == 0) {                                                                         \
-        if (threadIdx.x == 0) *a.st = s;                                                           \
+        if (threadIdx.x == 0) *a.st = *A.host = s;                                                 \
         t.clear_other_set();                                                                       \
     }
 
@@ -807,7 +808,7 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
 template <class P, int RS, int W>
 __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ ResArgs A)
 {
-    RES_PROLOGUE(P);
+    RES_PROLOGUE(P, sh.s.rro);
     const bool pre = !P::fp32 && A.p.pre;
     t.load_coefs(P::kx(a), P::ky(a), P::kz(a), P::mi(a, pre));
     t.load_operand(P::p(a));
@@ -916,7 +917,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
 template <class P, int RS, int W>
 __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__ ResArgs A)
 {
-    RES_PROLOGUE(P);
+    RES_PROLOGUE(P, P::fp32 ? sh.s.rro : sh.s.error);
     const bool pre = !P::fp32 && A.p.pre;
     t.load_coefs(P::kx(a), P::ky(a), P::kz(a), P::mi(a, pre));
     t.load_operand(P::u(a));
@@ -990,7 +991,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
 template <class P, int RS, int W>
 __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ ResArgs A)
 {
-    RES_PROLOGUE(P);
+    RES_PROLOGUE(P, sh.s.rro);
     t.load_coefs(a.kx, a.ky, a.kz, nullptr);
     t.load_operand(a.p[0]);
     constexpr bool PREG = RS <= 2;  // p waits in registers, else in its array, for the next outer iteration
@@ -1154,7 +1155,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
 template <class P, int RS, int W>
 __global__ void __launch_bounds__(32 * W, 1) k_res_jacobi(const __grid_constant__ ResArgs A)
 {
-    RES_PROLOGUE(P);
+    RES_PROLOGUE(P, sh.s.error);
     t.load_coefs(a.kx, a.ky, a.kz, nullptr);
     t.load_operand(a.u[0]);
     T un[RS][2];

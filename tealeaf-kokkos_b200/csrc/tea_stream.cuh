@@ -33,9 +33,10 @@ namespace tea {
 
 struct StreamArgs {
     FusedArgs f;
-    SolveState s0;  // the state the loop starts from (the final one goes to *f.st)
+    const SolveState* start;  // as in ResArgs
+    SolveState s0;
+    SolveState* host;
     SumArgs sum;
-    double scale;   // expected magnitude of the sums
     int seg;        // rows (2D) or planes (3D) of a work unit
 };
 
@@ -476,8 +477,8 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_con
     SolveState& s = sh.s;
     GridSum sum(A.sum, sh.sum);
     if (threadIdx.x == 0) {
-        s = A.s0;
-        sum.start(A.scale);
+        s = A.start ? *A.start : A.s0;
+        sum.start(s.rro);
     }
     constexpr int warps = ST_WARPS / StreamRing<T>::parts;  // that share a ring
     const int part = sum.warp / warps;
@@ -547,7 +548,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_con
         if (threadIdx.x == 0) {
             s.par_p = par;
             s.pending_p = s.pending_u = 1;
-            *a.st = s;
+            *a.st = *A.host = s;
         }
         sum.clear_other_set();
     }

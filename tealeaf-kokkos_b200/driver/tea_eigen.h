@@ -121,6 +121,14 @@ inline void tea_calc_ch_coefs(double* ch_alphas, double* ch_betas, double eigmin
         const double rho_new = 1.0 / (2.0 * sigma - rho_old);
         ch_alphas[k] = rho_new * rho_old;
         ch_betas[k] = 2.0 * rho_new / delta;
+        if (rho_new == rho_old) {
+            // The recurrence has reached its fixed point: every later entry is this one.
+            for (int j = k + 1; j < n; ++j) {
+                ch_alphas[j] = ch_alphas[k];
+                ch_betas[j] = ch_betas[k];
+            }
+            break;
+        }
         rho_old = rho_new;
     }
 }

@@ -91,6 +91,8 @@ struct RedScratch {
     DD* partials;           // [max_blocks * MAX_RED]
     unsigned int* counter;  // reset to 0 by the last block
     int max_blocks;
+    unsigned int* done;     // host memory: takes `ticket` once a result is in host memory (null: none)
+    unsigned int ticket;
 };
 
 template <int NV>
@@ -190,6 +192,11 @@ __device__ void grid_reduce(DDVec<NV> acc, const RedScratch& rs, double* out)
 #pragma unroll
         for (int k = 0; k < NV; ++k) out[k] = dd_value(b.v[k]);
         *rs.counter = 0u;
+        if (rs.done) {
+            // Every other block has ended its work: the host need not wait for the launch to retire.
+            __threadfence_system();
+            *(volatile unsigned int*)rs.done = rs.ticket;
+        }
     }
 }
 

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -145,8 +147,15 @@ Chunk* create_chunk(int nx, int ny, int nz, int rank)
     TEA_CK(cudaMalloc(&c->red.partials, sizeof(DD) * MAX_RED * c->red.max_blocks));
     TEA_CK(cudaMalloc(&c->red.counter, sizeof(unsigned int)));
     TEA_CK(cudaMemset(c->red.counter, 0, sizeof(unsigned int)));
-    TEA_CK(cudaHostAlloc(&c->h_out, 8 * sizeof(double), cudaHostAllocMapped));
+    // Eight results and, on a cache line of its own, the ticket of the last one.
+    TEA_CK(cudaHostAlloc(&c->h_out, 16 * sizeof(double), cudaHostAllocMapped));
     TEA_CK(cudaHostGetDevicePointer(&c->d_out, c->h_out, 0));
+    if (c->h_out) {
+        std::memset(c->h_out, 0, 16 * sizeof(double));
+        c->h_done = reinterpret_cast<volatile unsigned int*>(c->h_out + 8);
+    }
+    c->red.done = nullptr;
+    c->red.ticket = 0;
     TEA_CK(cudaDeviceSynchronize());
     if (rank == 0 && verbose()) {
         if (DIM == 2) std::printf("Problem Size: %dx%d\n", nx, ny);
@@ -174,10 +183,37 @@ void destroy_chunk(Chunk* c)
     delete c;
 }
 
+// The reduction scratch for a launch whose results the host waits for (await_result).
+RedScratch awaited(Chunk* c)
+{
+    ++c->red.ticket;
+    RedScratch rs = c->red;
+    rs.done = c->h_done ? reinterpret_cast<unsigned int*>(c->d_out + 8) : nullptr;
+    return rs;
+}
+
+// Waits for the results of the launch that got the last ticket.  The last block writes them and
+// then the ticket to host memory, which the host sees some 6 us before a stream synchronisation
+// would return; results that take longer than the spin, and launches that failed, are waited for
+// by a synchronisation, which also reports the error.
+void await_result(Chunk* c)
+{
+    TEA_CK(cudaGetLastError());
+    const unsigned int want = c->red.ticket;
+    const auto start = std::chrono::steady_clock::now();
+    while (c->h_done && *c->h_done != want) {
+        for (int k = 0; k < 64 && *c->h_done != want; ++k) {
+        }
+        if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(500)) break;
+    }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (!c->h_done || *c->h_done != want) sync(c);
+}
+
 // Result of a reduction kernel written through the mapped pointer.
 double result(Chunk* c, int k)
 {
-    sync(c);
+    await_result(c);
     c->d2h_bytes += sizeof(double);
     return ((volatile double*)c->h_out)[k];
 }
@@ -424,8 +460,8 @@ TEA_EXPORT void ext_field_summary_kernel_(const int* chunk, double* vol, double*
     Chunk* c = get_chunk(chunk);
     if (!c) return;
     k_field_summary<<<launch_blocks(c, c->inner.ntiles), dim3(TILE_X, TILE_Y), 0, c->stream>>>(
-        c->g, c->inner, c->f, c->red, c->d_out);
-    sync(c);
+        c->g, c->inner, c->f, awaited(c), c->d_out);
+    await_result(c);
     c->d2h_bytes += 4 * sizeof(double);
     volatile double* h = c->h_out;
     *vol = h[0];
@@ -557,7 +593,7 @@ TEA_EXPORT void ext_calculate_2norm_(const int* chunk, double* norm, const void*
     Chunk* c = get_chunk(chunk);
     if (!c) return;
     const double* b = *(const unsigned char*)normArray ? c->f.r : c->f.u0;
-    LAUNCH_PAIRS(k_2norm, c->g, b, c->red, c->d_out);
+    LAUNCH_PAIRS(k_2norm, c->g, b, awaited(c), c->d_out);
     *norm = result(c, 0);
 }
 
@@ -598,7 +634,7 @@ TEA_EXPORT void ext_jacobi_kernel_solve_(const int* chunk, double* error)
     Chunk* c = get_chunk(chunk);
     if (!c) return;
     k_jacobi_copy<<<pair_blocks(c), BLOCK, 0, c->stream>>>(c->g, c->f);
-    LAUNCH_PAIRS(k_jacobi_solve, c->g, c->f, c->red, c->d_out);
+    LAUNCH_PAIRS(k_jacobi_solve, c->g, c->f, awaited(c), c->d_out);
     *error = result(c, 0);
 }
 
@@ -616,7 +652,7 @@ TEA_EXPORT void ext_cg_solver_init_(const int* chunk, const int* coefficient, co
     const double rz = DIM == 3 ? *dt / (c->dz * c->dz) : 0.0;
     LAUNCH(k_cg_init_uw, c->full, c->g, c->full, c->f, *coefficient == 1 ? 1 : 0);
     LAUNCH(k_cg_init_k, c->skew, c->g, c->skew, c->f, rx, ry, rz);
-    LAUNCH(k_cg_calc_rro, c->inner, c->g, c->inner, c->f, c->preconditioner, c->red, c->d_out);
+    LAUNCH(k_cg_calc_rro, c->inner, c->g, c->inner, c->f, c->preconditioner, awaited(c), c->d_out);
     *rro = result(c, 0);
 }
 
@@ -624,7 +660,7 @@ TEA_EXPORT void ext_cg_calc_w_(const int* chunk, double* pw)
 {
     Chunk* c = get_chunk(chunk);
     if (!c) return;
-    LAUNCH_PAIRS(k_cg_calc_w, c->g, c->f, c->red, c->d_out);
+    LAUNCH_PAIRS(k_cg_calc_w, c->g, c->f, awaited(c), c->d_out);
     *pw = result(c, 0);
 }
 
@@ -632,7 +668,7 @@ TEA_EXPORT void ext_cg_calc_ur_(const int* chunk, const double* alpha, double* r
 {
     Chunk* c = get_chunk(chunk);
     if (!c) return;
-    LAUNCH_PAIRS(k_cg_calc_ur, c->g, c->f, *alpha, c->preconditioner, c->red, c->d_out);
+    LAUNCH_PAIRS(k_cg_calc_ur, c->g, c->f, *alpha, c->preconditioner, awaited(c), c->d_out);
     *rrn = result(c, 0);
 }
 

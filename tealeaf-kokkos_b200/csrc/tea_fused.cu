@@ -526,7 +526,11 @@ const void* res_kernel(int kind)
 {
     constexpr int RS = RES_FORMS[F].rows, W = RES_FORMS[F].warps;
     if constexpr (P::fp32) {
-        return kind == LOOP_CG32 ? (const void*)k_res_cg<P, RS, W> : (const void*)k_res_cheby<P, RS, W>;
+        switch (kind) {
+        case LOOP_CG32: return (const void*)k_res_cg<P, RS, W>;
+        case LOOP_PPCG32: return (const void*)k_res_ppcg<P, RS, W>;
+        default: return (const void*)k_res_cheby<P, RS, W>;
+        }
     } else {
         switch (kind) {
         case LOOP_CG: return (const void*)k_res_cg<P, RS, W>;
@@ -555,8 +559,8 @@ const void* res_kernel(int kind, int form)
 bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started)
 {
     const SolveState& s = *F->h_st;
-    const bool fp32 = kind == LOOP_CG32 || kind == LOOP_CHEBY32;
-    if (kind == LOOP_PPCG32 || (kind == LOOP_PPCG && s.precond)) return false;
+    const bool fp32 = kind == LOOP_CG32 || kind == LOOP_CHEBY32 || kind == LOOP_PPCG32;
+    if (kind == LOOP_PPCG && s.precond) return false;
     const ResPlan& p = fp32 ? F->res32 : F->res[(kind == LOOP_CG || kind == LOOP_CHEBY) && s.precond ? 1 : 0];
     if (p.blocks == 0 || s.par_u || s.par_p || s.pending_p || s.pending_u) return false;
     ResArgs A;
@@ -1012,12 +1016,12 @@ bool build_loop(Chunk* c, Fused* F, int kind, int inner_steps)
 }
 
 // The host record is pinned and the host rewrites it right after most pushes, so the copy
-// has read it before this returns.
-void push_state(Chunk* c, Fused* F)
+// has read it before this returns (without `wait`: before the pull_state that follows does).
+void push_state(Chunk* c, Fused* F, bool wait = true)
 {
     TEA_CK(cudaMemcpyAsync(F->d_st, F->h_st, sizeof(SolveState), cudaMemcpyHostToDevice, c->stream));
     c->h2d_bytes += sizeof(SolveState);
-    sync(c);
+    if (wait) sync(c);
 }
 
 void pull_state(Chunk* c, Fused* F)
@@ -1310,7 +1314,7 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
         bool converged = false;
         for (int guard = 0; !converged && guard < P->max_iters + 2; ++guard) {
             if (status_store().status == TEA_ERR_CUDA) break;
-            push_state(c, F);
+            push_state(c, F, false);
             stencil<OpOuterResid>(F, a, c->stream);
             pull_state(c, F);
             if (std::fabs(s.error) < eps || s.nonfinite) {

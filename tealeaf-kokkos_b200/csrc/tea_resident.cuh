@@ -1,6 +1,6 @@
 // On-chip iteration loops of the whole-solve path for grids that fit into the SMs' shared
 // memory and registers: one cooperative launch runs a whole loop (CG, Chebyshev, PPCG or
-// Jacobi, and the FP32 inner CG and Chebyshev solves) instead of a CUDA graph that launches
+// Jacobi, and the FP32 inner CG, Chebyshev and PPCG solves) instead of a CUDA graph that launches
 // one or more kernels per iteration.
 //
 // What bounds it.  On such grids a launch is all latency: reading the state, filling the
@@ -992,17 +992,17 @@ template <class P, int RS, int W>
 __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ ResArgs A)
 {
     RES_PROLOGUE(P, sh.s.rro);
-    t.load_coefs(a.kx, a.ky, a.kz, nullptr);
-    t.load_operand(a.p[0]);
-    constexpr bool PREG = RS <= 2;  // p waits in registers, else in its array, for the next outer iteration
+    t.load_coefs(P::kx(a), P::ky(a), P::kz(a), nullptr);
+    t.load_operand(P::p(a));
+    constexpr bool PREG = RS * sizeof(T) <= 16;  // p waits in registers, else in its array, for the next outer iteration
     T r[RS][2], w[RS][2], p[PREG ? RS : 1][2];
-    ResOwn<T, RS> u(t, a.u[0]);
+    ResOwn<T, RS> u(t, P::u(a));
 #pragma unroll
     for (int k = 0; k < RS; ++k) {
         r[k][0] = r[k][1] = w[k][0] = w[k][1] = (T)0;
         if (t.on(k)) {
-            ld_cells(a.r, t.gidx(k), r[k][0], r[k][1]);
-            if constexpr (PREG) ld_cells(a.p[0], t.gidx(k), p[k][0], p[k][1]);
+            ld_cells(P::r(a), t.gidx(k), r[k][0], r[k][1]);
+            if constexpr (PREG) ld_cells(P::p(a), t.gidx(k), p[k][0], p[k][1]);
         }
     }
     auto set_operand = [&](int k, T v0, T v1) {
@@ -1019,7 +1019,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
     bool lost = false;
     for (bool pend = false;; pend = true) {
         if (pend) {
-            const T beta = s.last_beta;
+            const T beta = (T)s.last_beta;
             ++t.tag;
             if constexpr (PREG) {
 #pragma unroll
@@ -1030,7 +1030,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
             } else {
 #pragma unroll
                 for (int k = 0; k < RS; ++k)
-                    if (t.on(k)) ld_cells(a.p[0], t.gidx(k), w[k][0], w[k][1]);
+                    if (t.on(k)) ld_cells(P::p(a), t.gidx(k), w[k][0], w[k][1]);
             }
 #pragma unroll
             for (int k = 0; k < RS; ++k)
@@ -1042,7 +1042,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                         p[k][0] = w[k][0];
                         p[k][1] = w[k][1];
                     } else {
-                        st_cells(a.p[0], t.gidx(k), t.both(), w[k][0], w[k][1]);
+                        st_cells(P::p(a), t.gidx(k), t.both(), w[k][0], w[k][1]);
                     }
                 }
             if (exchange() != RN_GO) break;
@@ -1051,21 +1051,17 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
         t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
             const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
             w[k][q] = wv;
-            t.add(acc, q, wv * nb.c);
+            t.add(acc, q, (double)wv * (double)nb.c);
         });
         if (t.reduce(
-                acc, 0, [] {},
-                [&](double v) {
-                    s.alpha = s.rro / v;
-                    return true;
-                },
+                acc, 0, [] {}, [&](double v) { return cg_after_pw(s, v); },
                 [&](double v) {
                     s.pw = v;
-                    if (blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
+                    if (!P::fp32 && blockIdx.x == 0) a.cg_alphas[s.n] = s.alpha;
                     if (!isfinite(v)) s.nonfinite = 1;
                 }) != RN_GO)
             break;
-        const T alpha = s.alpha, theta = s.theta;
+        const T alpha = (T)s.alpha, theta = (T)s.theta;
         ++t.tag;
 #pragma unroll
         for (int k = 0; k < RS; ++k)
@@ -1088,7 +1084,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
         if (exchange() != RN_GO) break;
         acc.hi = acc.lo = 0.0;
         for (int m = 1; m <= inner; ++m) {
-            const T al = a.ch_alphas[m - 1], be = a.ch_betas[m - 1];
+            const T al = (T)a.ch_alphas[m - 1], be = (T)a.ch_betas[m - 1];
             const bool last = m == inner;
             // u += sd first: its rows pass through w, which then takes the new sd.
             u.load(t, w);
@@ -1104,7 +1100,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                 const T rv = r[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
                 r[k][q] = rv;
                 w[k][q] = al * nb.c + be * rv;
-                if (last) t.add(acc, q, rv * rv);
+                if (last) t.add(acc, q, (double)rv * (double)rv);
             });
             if (last) break;
             __syncthreads();  // every warp has read the old sd
@@ -1122,15 +1118,22 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                 acc, 1, [] {},
                 [&](double v) {
                     s.last_beta = v / s.rro;
-                    s.rro = s.error = v;
-                    s.cheby_calc_steps = s.cheby_calc_steps + 1;
-                    end_iteration(a, s, PHASE_PPCG);
+                    s.rro = v;
+                    if constexpr (P::fp32) {
+                        s.n_inner = s.n_inner + 1;
+                        if (!isfinite(v)) s.inner_diverged = 1;  // the correction is dropped; CG takes over
+                        s.cont = isfinite(v) && v >= s.tol2 && s.n_inner < s.inner_max;
+                    } else {
+                        s.error = v;
+                        s.cheby_calc_steps = s.cheby_calc_steps + 1;
+                        end_iteration(a, s, PHASE_PPCG);
+                    }
                     return s.cont != 0;
                 },
                 [&](double v) {
                     s.rrn = v;
                     s.beta = s.last_beta;
-                    if (!isfinite(v)) s.nonfinite = 1;
+                    if (!P::fp32 && !isfinite(v)) s.nonfinite = 1;
                 }) != RN_GO)
             break;
     }
@@ -1143,8 +1146,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
     for (int k = 0; k < RS; ++k)
         if (t.on(k)) {
             const long i = t.gidx(k);
-            st_cells(a.r, i, t.both(), r[k][0], r[k][1]);
-            if constexpr (PREG) st_cells(a.p[0], i, t.both(), p[k][0], p[k][1]);
+            st_cells(P::r(a), i, t.both(), r[k][0], r[k][1]);
+            if constexpr (PREG) st_cells(P::p(a), i, t.both(), p[k][0], p[k][1]);
         }
     u.write(t);
     RES_EPILOGUE();

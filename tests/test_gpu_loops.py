@@ -74,7 +74,7 @@ def test_streaming_cg_equals_per_call(dim, shape, precond):
     _same(_run(deck, dim, fused=True), _run(deck, dim))
 
 
-@pytest.mark.parametrize("solver", ["cg", "chebyshev"])
+@pytest.mark.parametrize("solver", ["cg", "chebyshev", "ppcg"])
 @pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2] + STREAM_SHAPES[d][::2]])
 def test_one_launch_fp32_loops_equal_single_launches(dim, shape, solver):
     deck = _deck(dim, shape, solver, False)

@@ -401,10 +401,11 @@ void stencil(const Fused* F, const FusedArgs& a, cudaStream_t s)
     TEA_STENCIL<Op><<<F->stencil_blocks, TEA_STENCIL_BLOCK, 0, s>>>(a);
 }
 
-// The cheapest way to deal the grid to at most `sms` blocks, by a rough cost of one iteration in
-// nanoseconds: the row segments of the busiest warp, and with more than one block the waits for
-// the others and the halo cells.  blocks = 0 when no split fits.
-ResPlan res_plan(const Geom& g, int sms, int elem, bool pre, size_t smem)
+// The cheapest way to deal the grid to at most `sms` blocks, by a rough cost of half a CG iteration
+// in cycles: the row segments of the busiest warp, and with more than one block the waits for the
+// others and the halo cells.  Up to `cluster` blocks (0: no clusters) form a cluster where they
+// have a form for it.  blocks = 0 when no split fits.
+ResPlan res_plan(const Geom& g, int sms, int cluster, int elem, bool pre, size_t smem)
 {
     ResPlan best;
     double best_cost = 0.0;
@@ -422,23 +423,6 @@ ResPlan res_plan(const Geom& g, int sms, int elem, bool pre, size_t smem)
                 p.tw = std::min(g.nx, (xunits + nbx - 1) / nbx * 2);
                 p.th = (g.ny + nby - 1) / nby;
                 p.td = (g.nz + nbz - 1) / nbz;
-                // A strip's rows are dealt to as many warps as there are.
-                const long strips = (long)((p.tw + 63) / 64) * p.td;
-                int need = 0;
-                for (int form = 0; form < RES_FORM_COUNT; ++form) {
-                    const int warps = RES_FORMS[form].warps;
-                    if (strips > warps) continue;
-                    const int chunks = (int)std::min<long>(p.th, warps / strips);
-                    const int rows = (p.th + chunks - 1) / chunks;
-                    if (rows > RES_FORMS[form].rows) continue;
-                    need = rows;
-                    p.form = form;
-                    p.chunks = (p.th + rows - 1) / rows;
-                    break;
-                }
-                if (need == 0) continue;
-                p.warps = (int)strips * p.chunks;
-                if (p.blocks > 1 && p.warps < 2) p.warps = 2;
                 p.sx = even(p.tw + 4);
                 p.kxs = even(p.tw + 3);
                 p.tws = even(p.tw + 1);
@@ -450,21 +434,41 @@ ResPlan res_plan(const Geom& g, int sms, int elem, bool pre, size_t smem)
                 p.omi = p.okz + (d3 ? (p.td + 1) * p.th * p.tws : 0);
                 p.orh = p.omi + (pre ? p.td * p.th * p.tws : 0);
                 p.omh = p.orh + even(p.halo);
-                p.words = (p.omh + (pre ? even(p.halo) : 0) + 3) / 4 * 4;
-                p.bytes = (size_t)p.words * elem + (size_t)p.halo * sizeof(int2);
-                if (p.bytes > smem) continue;
-                const size_t own = (size_t)(p.td * p.th * p.tws + 3) / 4 * 4;
-                if (RES_FORMS[p.form].rows > 4 && p.bytes + own * elem <= smem) {
-                    p.ox = p.words;
-                    p.words += (int)own;
-                    p.bytes += own * elem;
-                }
-                const double cost =
-                    (p.form + 1 == RES_FORM_COUNT ? 600.0 : 300.0) * need * (0.4 + 0.6 * p.warps / RES_WARPS) +
-                    (p.blocks > 1 ? 1200.0 + 4.0 * p.blocks + 150.0 * p.halo / (32.0 * p.warps) : 0.0);
-                if (best.blocks == 0 || cost < best_cost) {
-                    best = p;
-                    best_cost = cost;
+                p.oh = p.omh + (pre ? even(p.halo) : 0);
+                p.hst = even(p.halo);
+                const ResPlan split = p;
+                // A strip's rows are dealt to as many warps as there are.
+                const long strips = (long)((p.tw + 63) / 64) * p.td;
+                for (int form = 0; form < RES_FORM_COUNT; ++form) {
+                    const int warps = RES_FORMS[form].warps;
+                    const bool cl = RES_FORMS[form].cluster;
+                    if (strips > warps || (cl && (p.blocks < 2 || p.blocks > cluster))) continue;
+                    const int chunks = (int)std::min<long>(p.th, warps / strips);
+                    const int rows = (p.th + chunks - 1) / chunks;
+                    if (rows > RES_FORMS[form].rows) continue;
+                    p = split;
+                    p.form = form;
+                    p.chunks = (p.th + rows - 1) / rows;
+                    p.warps = (int)strips * p.chunks;
+                    if (p.blocks > 1 && p.warps < 2) p.warps = 2;
+                    p.words = (p.oh + (cl ? 2 * p.hst : 0) + 3) / 4 * 4;
+                    p.bytes = (size_t)p.words * elem + (size_t)p.halo * sizeof(int2);
+                    if (p.bytes > smem) continue;
+                    const size_t own = (size_t)(p.td * p.th * p.tws + 3) / 4 * 4;
+                    if (RES_FORMS[form].rows > 4 && p.bytes + own * elem <= smem) {
+                        p.ox = p.words;
+                        p.words += (int)own;
+                        p.bytes += own * elem;
+                    }
+                    const double wait = p.blocks == 1 ? 0.0 : (cl ? 500.0 + 10.0 * p.blocks : 1200.0 + 4.0 * p.blocks);
+                    const double cost =
+                        (form + 1 == RES_FORM_COUNT ? 900.0 : 450.0) * rows * (0.4 + 0.6 * p.warps / RES_WARPS) + wait +
+                        (p.blocks > 1 ? 150.0 * p.halo / (32.0 * p.warps) : 0.0);
+                    if (best.blocks == 0 || cost < best_cost) {
+                        best = p;
+                        best_cost = cost;
+                    }
+                    break;
                 }
             }
     return best;
@@ -474,6 +478,23 @@ template <class K>
 void res_opt_in(K kernel, size_t bytes)
 {
     TEA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
+// A launch of one cluster of `blocks` blocks.
+void res_cluster_config(cudaLaunchConfig_t& L, cudaLaunchAttribute& at, const void* kernel, int blocks, int threads,
+                        size_t bytes, cudaStream_t stream)
+{
+    res_opt_in(kernel, bytes);
+    if (blocks > 8) TEA_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    L.gridDim = dim3(blocks);
+    L.blockDim = dim3(threads);
+    L.dynamicSmemBytes = bytes;
+    L.stream = stream;
+    L.attrs = &at;
+    L.numAttrs = 1;
 }
 
 // Grid and work units of the streamed CG loop: one block per SM, a unit per resident warp (2D)
@@ -511,9 +532,21 @@ void setup_resident(Chunk* c, Fused* F, int sms)
     setup_stream<ResF64>(F->stream, c->g, sms, smem);
     setup_stream<ResF32>(F->stream32, c->g, sms, smem);
     if ((size_t)c->g.nx * c->g.ny * c->g.nz > (size_t)sms * RES_WARPS * 8 * 64) return;
-    F->res[0] = res_plan(c->g, sms, sizeof(double), false, smem);
-    F->res[1] = res_plan(c->g, sms, sizeof(double), true, smem);
-    F->res32 = res_plan(c->g, sms, sizeof(float), false, smem);
+    // Clusters of 16 blocks where an SM group has that many SMs to give to this process, else of 8.
+    int cluster = RES_CLUSTER;
+    for (; cluster >= 8; cluster /= 2) {
+        const void* k = (const void*)k_res_cg<ResF64, 1, RES_WARPS, true>;
+        cudaLaunchConfig_t L = {};
+        cudaLaunchAttribute at = {};
+        res_cluster_config(L, at, k, cluster, 32 * RES_WARPS, smem, c->stream);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, k, &L) == cudaSuccess && n > 0) break;
+        cudaGetLastError();
+    }
+    if (cluster < 8) cluster = 0;
+    F->res[0] = res_plan(c->g, sms, cluster, sizeof(double), false, smem);
+    F->res[1] = res_plan(c->g, sms, cluster, sizeof(double), true, smem);
+    F->res32 = res_plan(c->g, sms, cluster, sizeof(float), false, smem);
     if (F->res[0].blocks == 0 && F->res32.blocks == 0) return;
     const size_t rim = 2 * c->field_elems * sizeof(ResWord);
     TEA_CK(cudaMalloc(&F->rim, rim));
@@ -525,31 +558,33 @@ template <class P, int F>
 const void* res_kernel(int kind)
 {
     constexpr int RS = RES_FORMS[F].rows, W = RES_FORMS[F].warps;
+    constexpr bool CL = RES_FORMS[F].cluster;
     if constexpr (P::fp32) {
         switch (kind) {
-        case LOOP_CG32: return (const void*)k_res_cg<P, RS, W>;
-        case LOOP_PPCG32: return (const void*)k_res_ppcg<P, RS, W>;
-        default: return (const void*)k_res_cheby<P, RS, W>;
+        case LOOP_CG32: return (const void*)k_res_cg<P, RS, W, CL>;
+        case LOOP_PPCG32: return (const void*)k_res_ppcg<P, RS, W, CL>;
+        default: return (const void*)k_res_cheby<P, RS, W, CL>;
         }
     } else {
         switch (kind) {
-        case LOOP_CG: return (const void*)k_res_cg<P, RS, W>;
-        case LOOP_CHEBY: return (const void*)k_res_cheby<P, RS, W>;
-        case LOOP_PPCG: return (const void*)k_res_ppcg<P, RS, W>;
-        default: return (const void*)k_res_jacobi<P, RS, W>;
+        case LOOP_CG: return (const void*)k_res_cg<P, RS, W, CL>;
+        case LOOP_CHEBY: return (const void*)k_res_cheby<P, RS, W, CL>;
+        case LOOP_PPCG: return (const void*)k_res_ppcg<P, RS, W, CL>;
+        default: return (const void*)k_res_jacobi<P, RS, W, CL>;
         }
     }
 }
 template <class P>
 const void* res_kernel(int kind, int form)
 {
-    static_assert(RES_FORM_COUNT == 5, "every form has its kernels");
+    static_assert(RES_FORM_COUNT == 6, "every form has its kernels");
     switch (form) {
     case 0: return res_kernel<P, 0>(kind);
     case 1: return res_kernel<P, 1>(kind);
     case 2: return res_kernel<P, 2>(kind);
     case 3: return res_kernel<P, 3>(kind);
-    default: return res_kernel<P, 4>(kind);
+    case 4: return res_kernel<P, 4>(kind);
+    default: return res_kernel<P, 5>(kind);
     }
 }
 
@@ -574,9 +609,18 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started
     A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->m_st)};
     A.epoch = F->epoch;
     const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
-    res_opt_in(k, p.bytes);
     void* args[] = {&A};
-    if (cudaLaunchCooperativeKernel(k, dim3(p.blocks), dim3(32 * p.warps), args, p.bytes, c->stream) != cudaSuccess) {
+    cudaError_t launched;
+    if (RES_FORMS[p.form].cluster) {
+        cudaLaunchConfig_t L = {};
+        cudaLaunchAttribute at = {};
+        res_cluster_config(L, at, k, p.blocks, 32 * p.warps, p.bytes, c->stream);
+        launched = cudaLaunchKernelExC(&L, k, args);
+    } else {
+        res_opt_in(k, p.bytes);
+        launched = cudaLaunchCooperativeKernel(k, dim3(p.blocks), dim3(32 * p.warps), args, p.bytes, c->stream);
+    }
+    if (launched != cudaSuccess) {
         // Fewer SMs than the device reports (a partition of it): the loops run as graphs.
         cudaGetLastError();
         F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;

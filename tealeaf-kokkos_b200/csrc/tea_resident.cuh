@@ -28,15 +28,23 @@
 //
 // Sums.  An all-to-all of the blocks' double-double partials through such words took 2400-2900
 // cycles at 64-128 blocks, a counter that all blocks add to and poll 1400-1550 (148 blocks),
-// so a dot product is formed by integer atomics: each thread's partial is cut into five 22-bit
+// so a dot product is formed by integer atomics: each thread's partial is cut into four 26-bit
 // limbs at bit positions that all blocks know (from the last value of the same sum), the
 // limbs add up exactly in any order, and each limb's 64-bit word counts its arrivals in
 // its top byte, so that the poll that sees the last arrival has the sum.  The integer sums
-// also replace five levels of double-double merges in a warp by five redux instructions.
+// also replace five levels of double-double merges in a warp by four redux instructions.
+// (Five 22-bit limbs, which 32 bits could sum over a block, and a chain of double-double adds
+// behind the poll cost 3 % of an iteration more.)
 // Every block then forms the rounded value and runs the scalar recurrence and the loop test
-// itself.  A thread's partial is kept to 2^-89 of the sum's last value: rounded, the sums are
+// itself.  A thread's partial is kept to 2^-95 of the sum's last value: rounded, the sums are
 // those of the per-launch kernels' double-double bit for bit, and per cell the operations and
 // their order are those of the per-call kernels.
+//
+// Clusters.  Up to 16 blocks with one row a warp (some 16000 cells) form one cluster: limbs and rim
+// values go straight into the other blocks' shared memory, and an mbarrier there counts their
+// bytes.  The rim buffers and the limbs' slots are double-buffered as above.  A CG iteration
+// takes 2.6 us at 64^2 and 3.0 at 128^2 (through L2 3.9), a Jacobi one 1.5 and 1.9 (2.1), a
+// Chebyshev one 1.0 and 1.2 (1.4).
 //
 // Every poll is bounded; a block that gives up raises a flag that ends the other blocks'
 // polls too, and the host reports the solve as failed.
@@ -49,14 +57,21 @@
 namespace tea {
 
 constexpr int RES_WARPS = 16;  // most warps of a block
-// The kernels' forms: at most RS rows a warp, W warps a block.
+// The kernels' forms: at most RS rows a warp, W warps a block; the blocks of the cluster form are one
+// cluster, which exchanges through its shared memory.  It has one row a warp: with two, in 16 blocks,
+// CG takes as long as with one in twice the blocks (3.65 us an iteration at 160^2 either way), and
+// Chebyshev longer (1.67 against 1.42).
 struct ResForm {
     int rows, warps;
+    bool cluster;
 };
-constexpr ResForm RES_FORMS[] = {{1, 16}, {2, 16}, {4, 16}, {8, 12}, {8, 16}};
-constexpr int RES_FORM_COUNT = 5;
+constexpr ResForm RES_FORMS[] = {{1, 16, true},  {1, 16, false}, {2, 16, false},
+                                 {4, 16, false}, {8, 12, false}, {8, 16, false}};
+constexpr int RES_FORM_COUNT = 6;
+constexpr int RES_CLUSTER = 16;  // most blocks of a cluster
+constexpr int RES_TRIES = 1 << 18;  // tries at an mbarrier before a wait gives up
 constexpr int RES_POLLS = 1 << 21;  // rounds of polls before a wait gives up (a second or two)
-constexpr int RES_LIMBS = 5;         // limbs of a sum, and one word of flags
+constexpr int RES_LIMBS = 4;         // limbs of a sum, and one word of flags
 constexpr int RES_SUM_STRIDE = 32;   // 64-bit words between two sums: a sum's words share a line
 constexpr int RES_SUM_WORDS = 2 * 2 * RES_SUM_STRIDE;  // two sets of two parities
 
@@ -77,6 +92,7 @@ struct ResPlan {
     int pre = 0;              // with the preconditioner's diagonal
     int okx = 0, oky = 0, okz = 0, omi = 0, orh = 0, omh = 0;  // first elements of Kx, Ky, Kz, mi, halo r, halo mi
     int ox = 0;               // ... of one more vector of the loop, where there is room (else 0)
+    int oh = 0, hst = 0;      // cluster: first element of the two buffers that the neighbours fill, and their stride
     int words = 0;            // elements of T before the halo table
     size_t bytes = 0;         // dynamic shared memory
 };
@@ -148,13 +164,85 @@ __device__ __forceinline__ double res_value<double>(unsigned long long b) { retu
 template <>
 __device__ __forceinline__ float res_value<float>(unsigned long long b) { return __uint_as_float((unsigned)b); }
 
+// ------------------------------------------------------------------ clusters
+
+__device__ __forceinline__ unsigned res_shared(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+// The address in block `rank` of the cluster of what lies at `a` in this block.
+__device__ __forceinline__ unsigned res_remote(unsigned a, int rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+// Stores that count their bytes at an mbarrier of the block that they go to.
+__device__ __forceinline__ void res_send(unsigned a, unsigned bar, double v)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
+                 "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void res_send(unsigned a, unsigned bar, float v)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(a),
+                 "r"(__float_as_uint(v)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void res_send(unsigned a, unsigned bar, unsigned long long v0, unsigned long long v1)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(a), "l"(v0),
+                 "l"(v1), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void res_expect(unsigned bar, int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool res_arrived(unsigned bar, unsigned phase)
+{
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(bar), "r"(phase)
+        : "memory");
+    return ok != 0;
+}
+// Waits for a phase of an mbarrier; gives up as res_wait does.
+__device__ __forceinline__ void res_wait_bar(unsigned bar, unsigned phase, int* fail, bool& gave_up)
+{
+    for (int k = 0; !res_arrived(bar, phase); ++k)
+        if ((k & 1023) == 1023 && (k >= RES_TRIES || *(volatile int*)fail != 0)) {
+            gave_up = true;
+            break;
+        }
+}
+__device__ __forceinline__ void res_cluster_sync()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+
+// What the blocks of a cluster write into each other: the blocks' limbs of a sum (by the sum's
+// parity), and per face that a tile shares the neighbour's buffer and mbarriers.
+struct ResFace {
+    unsigned data, bar;
+};
+template <bool CL>
+struct ClusterShared {
+    alignas(16) unsigned long long sums[2][RES_CLUSTER][4];
+    unsigned long long sum_bar[2], rim_bar[2];
+    ResFace face[6];
+};
+template <>
+struct ClusterShared<false> {
+};
+
 // ------------------------------------------------------------------ sums
 
 // Limb positions of a sum, from the biased exponent E of its expected magnitude m: a thread's
-// partial may reach 2^8 m, the limbs are 22 bits apart (so that a block's total of a limb is
-// below 2^31), the first one's unit is 2^-13 m and the last one's 2^-101 m.
-constexpr int RES_E_MIN = 130, RES_E_MAX = 1980;  // expected exponents stay inside (units are normal numbers)
-constexpr int RES_E_UNIT = -13, RES_E_STEP = 22, RES_E_ROOM = 7;
+// partial may reach 2^8 m, the limbs are 26 bits apart (so that a warp's total of a limb is
+// at most 2^30), the first one's unit is 2^-17 m and the last one's 2^-95 m.
+constexpr int RES_E_MIN = 97, RES_E_MAX = 1980;  // expected exponents stay inside (units are normal numbers)
+constexpr int RES_E_UNIT = -17, RES_E_STEP = 26, RES_E_ROOM = 7;
 constexpr int RES_E_LOST = 10;  // a sum this far below the expected magnitude is formed again
 
 __device__ __forceinline__ int res_exponent(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
@@ -165,8 +253,8 @@ __device__ __forceinline__ double res_unit(int E, int limb)
 }
 
 // A lane's partial hi + lo cut into limbs: 1.5 * 2^52 units plus the rest has the limb in its
-// low word.  lo, below 2^-43 m, joins after the second limb, whose rest is below 2^-36 m: what
-// that sum rounds off is below 2^-89 m.
+// low word.  lo, below 2^-44 m, joins after the second limb, whose rest is at most 2^-44 m: what
+// that sum rounds off is below 2^-95 m.
 __device__ __forceinline__ void res_limbs(double hi, double lo, int E, int (&v)[RES_LIMBS])
 {
     double rest = hi;
@@ -180,25 +268,29 @@ __device__ __forceinline__ void res_limbs(double hi, double lo, int E, int (&v)[
     }
 }
 
-struct SumShared {
+template <bool CL = false>
+struct SumShared : ClusterShared<CL> {
     int limbs[RES_LIMBS][RES_WARPS];
     int scale[2];  // expected exponents of the loop's two sums
     int bad;       // a partial out of range (1) or not finite (2)
     int next;      // what follows a sum or an iteration: RN_*
+    int lost;      // a wait of this block has given up
     double sum;    // the last sum
 };
 enum { RN_GO = 0, RN_STOP = 1, RN_AGAIN = 2, RN_FAIL = 4 };
 
 // A block's part in the sums over the grid.
+template <bool CL = false>
 struct GridSum {
     const SumArgs& sa;
-    SumShared& ss;
+    SumShared<CL>& ss;
     int nw, warp, lane;
     unsigned long long seen0 = 0, seen1 = 0;  // this lane's word of the sums, as last read, by parity
     int parity = 0;
+    unsigned phases = 0;  // of the cluster's sum barriers, a bit for each parity
     bool gave_up = false;
 
-    __device__ __forceinline__ GridSum(const SumArgs& a, SumShared& s)
+    __device__ __forceinline__ GridSum(const SumArgs& a, SumShared<CL>& s)
         : sa(a), ss(s), nw(blockDim.x >> 5), warp(threadIdx.x >> 5), lane(threadIdx.x & 31)
     {
     }
@@ -207,6 +299,7 @@ struct GridSum {
         ss.scale[0] = ss.scale[1] = res_clamp(res_exponent(scale));
         ss.bad = 0;
         ss.next = RN_GO;
+        ss.lost = 0;
     }
     // The other set's words, by one block at the end of the launch.
     __device__ __forceinline__ void clear_other_set() const
@@ -240,23 +333,29 @@ struct GridSum {
             parity ^= 1;
             __syncthreads();
             if (warp == 0) {
-                long long mine = 0;
+                unsigned bad = ss.bad;
+                long long tot[RES_LIMBS];
 #pragma unroll
                 for (int i = 0; i < RES_LIMBS; ++i) {
-                    const int w = __reduce_add_sync(0xffffffffu, lane < nw ? ss.limbs[i][lane] : 0);
-                    if (lane == i) mine = w;
+                    // The halves of the warps' limbs apart: together they may exceed 32 bits.
+                    const int v = lane < nw ? ss.limbs[i][lane] : 0;
+                    const int low = __reduce_add_sync(0xffffffffu, v & 0xffff), high = __reduce_add_sync(0xffffffffu, v >> 16);
+                    tot[i] = (long long)high * 65536 + low;
                 }
-                unsigned bad = ss.bad;
                 const int nb = sa.blocks;
-                if (nb > 1) {
-                    // A count in the top byte; below it the limb, raised to be positive.  The warp
-                    // stays together: a lane that polled before another has added would wait
-                    // for a word that the other blocks' same lanes wait for too.  The atomics
-                    // return a value so that the polls begin when this block's have arrived
-                    // (1550 cycles a sum against 2050 at 64 blocks).
-                    constexpr long long bias = 1ll << 32;
+                constexpr long long bias = 1ll << 36;  // raises a block's limbs to be positive
+                if constexpr (CL) {
+                    all_to_all(tot, bad, nb, bias);
+                } else if (nb > 1) {
+                    // A count in the top byte; below it the limb.  The warp stays together: a lane
+                    // that polled before another has added would wait for a word that the other
+                    // blocks' same lanes wait for too.  The atomics return a value so that the
+                    // polls begin when this block's have arrived (1550 cycles a sum against 2050
+                    // at 64 blocks).
                     const bool has = lane <= RES_LIMBS;
-                    mine = lane == RES_LIMBS ? (long long)((bad & 1) + ((bad & 2) << 15)) : mine;
+                    long long mine = (long long)((bad & 1) + ((bad & 2) << 15));
+#pragma unroll
+                    for (int i = 0; i < RES_LIMBS; ++i) mine = lane == i ? tot[i] : mine;
                     unsigned long long* q =
                         sa.sums + (sa.set * 2 + parity) * RES_SUM_STRIDE + (has ? lane : RES_LIMBS);
                     const unsigned long long add = (1ull << 56) + (unsigned long long)(mine + bias);
@@ -277,15 +376,19 @@ struct GridSum {
                     mine = (long long)((now - old) & ((1ull << 56) - 1)) - nb * bias;
                     seen0 = parity ? seen0 : now;
                     seen1 = parity ? now : seen1;
+#pragma unroll
+                    for (int i = 0; i < RES_LIMBS; ++i) tot[i] = __shfl_sync(0xffffffffu, mine, i);
                     bad = (unsigned)__shfl_sync(0xffffffffu, (int)mine, RES_LIMBS);
                     bad = ((bad & 0xffff) ? 1 : 0) | ((bad >> 16) ? 2 : 0);
                 }
-                const double part = (double)mine * res_unit(E, lane < RES_LIMBS ? lane : 0);
-                DD s = {part, 0.0};
-#pragma unroll
-                for (int i = 1; i < RES_LIMBS; ++i) dd_add(s, __shfl_sync(0xffffffffu, part, i));
+                // Each total is below 2^53, so exact; the two low limbs' sum is rounded at 2^-89 m
+                // unless the partials of 2^16 threads all end in the same way.
+                static_assert(RES_LIMBS == 4, "the limbs summed here");
+                DD s = {(double)tot[0] * res_unit(E, 0), 0.0};
+                dd_add(s, (double)tot[1] * res_unit(E, 1));
+                const double low = (double)tot[2] * res_unit(E, 2) + (double)tot[3] * res_unit(E, 3);
                 if (lane == 0) {
-                    double sum = dd_value(s);
+                    double sum = s.hi + (s.lo + low);
                     int e = res_clamp(res_exponent(sum)), next = RN_GO;
                     if (bad & 2) {
                         sum = CUDART_NAN;
@@ -315,12 +418,50 @@ struct GridSum {
             }
         }
     }
+    // The limbs and flags of all blocks of the cluster: each block sends its own to every block.
+    __device__ __forceinline__ void all_to_all(long long (&tot)[RES_LIMBS], unsigned& bad, int nb, long long bias)
+    {
+        if constexpr (CL) {
+            const unsigned bar = res_shared(&ss.sum_bar[parity]);
+            if (lane == 0) res_expect(bar, 32 * nb);
+            if (lane < nb) {
+                const unsigned to = res_remote(res_shared(&ss.sums[parity][blockIdx.x][0]), lane), at = res_remote(bar, lane);
+                res_send(to, at, (unsigned long long)(tot[0] + bias) | (unsigned long long)bad << 56,
+                         (unsigned long long)(tot[1] + bias));
+                res_send(to + 16, at, (unsigned long long)(tot[2] + bias), (unsigned long long)(tot[3] + bias));
+            }
+            __syncwarp();
+            res_wait_bar(bar, phases >> parity & 1, sa.fail, gave_up);
+            phases ^= 1u << parity;
+            unsigned flags = 0;
+            long long v[RES_LIMBS] = {0, 0, 0, 0};
+            if (lane < nb) {
+                const ulonglong2 *q = reinterpret_cast<const ulonglong2*>(&ss.sums[parity][lane][0]), a = q[0], b = q[1];
+                flags = (unsigned)(a.x >> 56);
+                v[0] = (long long)(a.x & ((1ull << 56) - 1)) - bias;
+                v[1] = (long long)a.y - bias;
+                v[2] = (long long)b.x - bias;
+                v[3] = (long long)b.y - bias;
+            }
+            bad = __reduce_or_sync(0xffffffffu, flags);
+#pragma unroll
+            for (int i = 0; i < RES_LIMBS; ++i) {
+                const int low = __reduce_add_sync(0xffffffffu, (int)(v[i] & 0xfffff)),
+                          high = __reduce_add_sync(0xffffffffu, (int)(v[i] >> 20));
+                tot[i] = (long long)high * (1 << 20) + low;
+            }
+        }
+    }
     // The end of an exchange: after it every thread sees what the others have written and what
     // warp 0 has decided.
     __device__ __forceinline__ int finish()
     {
-        if (gave_up) *(volatile int*)sa.fail = 1;
-        return __syncthreads_or(gave_up) ? RN_FAIL : ss.next;
+        if (gave_up) {
+            *(volatile int*)sa.fail = 1;
+            ss.lost = 1;
+        }
+        __syncthreads();
+        return ss.lost ? RN_FAIL : ss.next;
     }
 };
 
@@ -347,16 +488,26 @@ enum {
     RF_XM = 4, RF_XP0 = 8, RF_XP1 = 16,  // an x-neighbour is the cell itself (domain face)
     RF_P0 = 32, RF_P1 = 64,              // the cells of every row lie on the tile's rim
     RF_PFIRST = 128, RF_PLAST = 256,     // the first (last) row's do
-    RF_WFIRST = 512, RF_WLAST = 1024     // the row below the first (above the last) is itself
+    RF_WFIRST = 512, RF_WLAST = 1024,    // the row below the first (above the last) is itself
+    // Cluster forms: the neighbours that the cells go to besides those of the first and last row.
+    RF_SXM = 2048, RF_SX0 = 4096, RF_SX1 = 8192, RF_SZM = 16384, RF_SZP = 32768
 };
 
+template <bool CL>
 struct ResShared {
     SolveState s;
-    SumShared sum;
+    SumShared<CL> sum;
 };
 
-template <class T, int RS>
-struct ResTile : GridSum {
+template <class T, int RS, bool CL>
+struct ResTile : GridSum<CL> {
+    using Base = GridSum<CL>;
+    using Base::gave_up;
+    using Base::lane;
+    using Base::nw;
+    using Base::sa;
+    using Base::ss;
+    using Base::warp;
     const ResArgs& A;
     const Geom& g;
     T* const V;   // shared memory: the operand, then the arrays at the plan's offsets
@@ -371,8 +522,8 @@ struct ResTile : GridSum {
     int dzm, dzp;          // offsets of the z-neighbours (0 at a domain face)
     unsigned long long tag;   // epoch of the last rim exchange
 
-    __device__ __forceinline__ ResTile(const ResArgs& a, ResShared& s, T* mem)
-        : GridSum(a.sum, s.sum), A(a), g(a.f.g), V(mem)
+    __device__ __forceinline__ ResTile(const ResArgs& a, ResShared<CL>& s, T* mem)
+        : Base(a.sum, s.sum), A(a), g(a.f.g), V(mem)
     {
         const ResPlan& p = a.p;
         const int b = blockIdx.x;
@@ -385,7 +536,7 @@ struct ResTile : GridSum {
         td = res_split(g.nz, 1, bz + 1, p.nbz) - z0;
         sx = p.sx;
         plane = (th + 2) * sx;
-        tag = a.epoch;
+        tag = CL ? 0 : a.epoch;
         // The warp's strip, plane and rows.
         const int strips = (tw + 63) / 64;
         const int strip = warp % strips, rest = warp / strips;
@@ -404,6 +555,9 @@ struct ResTile : GridSum {
              (a1 && (zrim || (x + 1 == tw - 1 && !xr)) ? RF_P1 : 0) | (y == 0 && y0 > 0 ? RF_PFIRST : 0) |
              (y + rows == th && y0 + th < g.ny ? RF_PLAST : 0) | (y == 0 && y0 == 0 ? RF_WFIRST : 0) |
              (y + rows == th && y0 + th == g.ny ? RF_WLAST : 0);
+        if (CL && a0)
+            fl |= (x == 0 && !xl ? RF_SXM : 0) | (x == tw - 1 && !xr ? RF_SX0 : 0) | (x + 1 == tw - 1 && !xr ? RF_SX1 : 0) |
+                  (z == 0 && z0 > 0 ? RF_SZM : 0) | (z == td - 1 && z0 + td < g.nz ? RF_SZP : 0);
         dzm = z == 0 && z0 == 0 ? 0 : plane;
         dzp = z == td - 1 && z0 + td == g.nz ? 0 : plane;
         const int row = z * th + y;
@@ -413,6 +567,44 @@ struct ResTile : GridSum {
         okz = p.okz + row * p.tws + x;
         gi = fidx(g, HALO_PAD + x0 + x, HALO_PAD + y0 + y, DIM == 3 ? HALO_PAD + z0 + z : 0);
         build_table();
+        if constexpr (CL) join(bx, by, bz);
+    }
+    // Set up the block's mbarriers and what it needs to know of its neighbours' buffers.
+    __device__ void join(int bx, int by, int bz)
+    {
+        if constexpr (CL) {
+            const ResPlan& p = A.p;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < 2; ++k) {
+                    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(res_shared(&ss.sum_bar[k])) : "memory");
+                    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(res_shared(&ss.rim_bar[k])) : "memory");
+                }
+                asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            }
+            if (threadIdx.x < 6) {
+                // The neighbour at face f sees this tile at its face f ^ 1.
+                const int f = threadIdx.x, d = (f & 1) ? 1 : -1;
+                const int nx = bx + (f >> 1 == 0 ? d : 0), ny = by + (f >> 1 == 1 ? d : 0), nz = bz + (f >> 1 == 2 ? d : 0);
+                if (nx >= 0 && nx < p.nbx && ny >= 0 && ny < p.nby && nz >= 0 && nz < p.nbz) {
+                    const int w = res_split(g.nx, 2, nx + 1, p.nbx) - res_split(g.nx, 2, nx, p.nbx);
+                    const int h = res_split(g.ny, 1, ny + 1, p.nby) - res_split(g.ny, 1, ny, p.nby);
+                    const int e = res_split(g.nz, 1, nz + 1, p.nbz) - res_split(g.nz, 1, nz, p.nbz);
+                    int base = 0;
+                    for (int q = 0; q < (f ^ 1); ++q) base += face_cells(q, nx, ny, nz, w, h, e);
+                    const int rank = (nz * p.nby + ny) * p.nbx + nx;
+                    ss.face[f].data = res_remote(res_shared(V + p.oh + base), rank);
+                    ss.face[f].bar = res_remote(res_shared(&ss.rim_bar[0]), rank);
+                }
+            }
+            res_cluster_sync();
+        }
+    }
+    // Halo cells at face f of the tile of block (bx, by, bz), w x h x e cells.
+    __device__ __forceinline__ int face_cells(int f, int bx, int by, int bz, int w, int h, int e) const
+    {
+        const int at = f >> 1 == 0 ? bx : (f >> 1 == 1 ? by : bz), n = f >> 1 == 0 ? A.p.nbx : (f >> 1 == 1 ? A.p.nby : A.p.nbz);
+        if ((f & 1) ? at == n - 1 : at == 0) return 0;
+        return f >> 1 == 0 ? h * e : (f >> 1 == 1 ? w * e : w * h);
     }
 
     __device__ __forceinline__ bool on(int k) const { return (fl & RF_A0) && k < rows; }
@@ -543,8 +735,12 @@ struct ResTile : GridSum {
                 ky0 = ky1;
             }
     }
-    // Adds a product to a thread's sum; the second cell of a row may not exist.
-    __device__ __forceinline__ void add(DD& acc, int q, double v) const { dd_add(acc, q == 0 || both() ? v : 0.0); }
+    // Adds cell q of row k to a thread's sum; the second cell of a row may not exist.
+    __device__ __forceinline__ void add(DD& acc, int k, int q, double v) const
+    {
+        if (k == 0 && q == 0) acc.hi = v;
+        else dd_add(acc, q == 0 || both() ? v : 0.0);
+    }
 
     __device__ __forceinline__ void store(int k, T v0, T v1) const
     {
@@ -552,9 +748,46 @@ struct ResTile : GridSum {
         if (both()) st_two(cell(k), v0, v1);
         else *cell(k) = v0;
     }
+    // The next rim exchange.  In a cluster it is counted from 1, and fills buffer (tag - 1) & 1.
+    __device__ __forceinline__ void next_exchange()
+    {
+        ++tag;
+        if constexpr (CL)
+            if (threadIdx.x == 0) res_expect(res_shared(&ss.rim_bar[turn()]), nh * (int)sizeof(T));
+    }
+    __device__ __forceinline__ int turn() const { return (int)(tag - 1) & 1; }
+    __device__ __forceinline__ void send(int f, int i, T v) const
+    {
+        if constexpr (CL) {
+            const ResFace q = ss.face[f];
+            res_send(q.data + (turn() * A.p.hst + i) * (int)sizeof(T), q.bar + 8 * turn(), v);
+        }
+    }
     // Publish the rim cells of row k under the current exchange's epoch.
     __device__ __forceinline__ void publish(int k, T v0, T v1) const
     {
+        if constexpr (CL) {
+            const int ix = z * th + y + k, iy = z * tw + x, iz = (y + k) * tw + x;
+            if (fl & RF_SXM) send(0, ix, v0);
+            if (fl & (RF_SX0 | RF_SX1)) send(1, ix, (fl & RF_SX0) ? v0 : v1);
+            if (k == 0 && (fl & RF_PFIRST)) {
+                send(2, iy, v0);
+                if (both()) send(2, iy + 1, v1);
+            }
+            if (k == rows - 1 && (fl & RF_PLAST)) {
+                send(3, iy, v0);
+                if (both()) send(3, iy + 1, v1);
+            }
+            if (DIM == 3 && (fl & RF_SZM)) {
+                send(4, iz, v0);
+                if (both()) send(4, iz + 1, v1);
+            }
+            if (DIM == 3 && (fl & RF_SZP)) {
+                send(5, iz, v0);
+                if (both()) send(5, iz + 1, v1);
+            }
+            return;
+        }
         int rim = fl & (RF_P0 | RF_P1);
         if ((k == 0 && (fl & RF_PFIRST)) || (k == rows - 1 && (fl & RF_PLAST))) rim = RF_P0 | (both() ? RF_P1 : 0);
         if (rim) {
@@ -569,6 +802,13 @@ struct ResTile : GridSum {
     __device__ __forceinline__ void collect(int first, F&& put)
     {
         if (nh == 0 || warp < first) return;
+        if constexpr (CL) {
+            const int h0 = (warp - first) * 32 + lane;
+            if (h0 >= nh) return;
+            res_wait_bar(res_shared(&ss.rim_bar[turn()]), (unsigned)(tag - 1) >> 1 & 1, sa.fail, gave_up);
+            for (int h = h0; h < nh; h += (nw - first) * 32) put(h, V[A.p.oh + turn() * A.p.hst + h]);
+            return;
+        }
         const ResWord* q = A.rim + (tag & 1) * A.elems + kLeadPad;
         for (int h = (warp - first) * 32 + lane; h < nh; h += (nw - first) * 32) {
             put(h, res_value<T>(res_wait(q + table()[h].y, tag, sa.fail, gave_up)));
@@ -623,12 +863,12 @@ __device__ __forceinline__ void st_cells(T* a, long i, bool both, T x, T y)
 // side.  Up to four rows of it stay in registers; with more rows the two vectors that are live
 // across a sum fill the registers, and it lies in shared memory where there is room, else in
 // L2, from which all rows are loaded before any is stored.
-template <class T, int RS>
+template <class T, int RS, bool CL>
 struct ResOwn {
     static constexpr bool kept = RS * sizeof(T) <= 32;
     T v[kept ? RS : 1][2];
     T* far;  // the array
-    __device__ __forceinline__ ResOwn(const ResTile<T, RS>& t, T* array) : far(array)
+    __device__ __forceinline__ ResOwn(const ResTile<T, RS, CL>& t, T* array) : far(array)
     {
 #pragma unroll
         for (int k = 0; k < RS; ++k)
@@ -642,7 +882,7 @@ struct ResOwn {
             }
     }
     // The rows, in `w` when they are not kept.
-    __device__ __forceinline__ void load(const ResTile<T, RS>& t, T (&w)[RS][2]) const
+    __device__ __forceinline__ void load(const ResTile<T, RS, CL>& t, T (&w)[RS][2]) const
     {
         if constexpr (kept) {
 #pragma unroll
@@ -660,7 +900,7 @@ struct ResOwn {
                 }
         }
     }
-    __device__ __forceinline__ void store(const ResTile<T, RS>& t, const T (&w)[RS][2])
+    __device__ __forceinline__ void store(const ResTile<T, RS, CL>& t, const T (&w)[RS][2])
     {
         if constexpr (kept) {
 #pragma unroll
@@ -678,7 +918,7 @@ struct ResOwn {
         }
     }
     // Back to the array at the end of a loop that updates it.
-    __device__ __forceinline__ void write(const ResTile<T, RS>& t) const
+    __device__ __forceinline__ void write(const ResTile<T, RS, CL>& t) const
     {
 #pragma unroll
         for (int k = 0; k < RS; ++k)
@@ -719,11 +959,11 @@ __device__ __forceinline__ T res_smvp(T d, const NbT<T>& a, T kx0, T kx1, T ky0,
 
 // Diagonals of the warp's cells: in registers where there is room, else formed again from the
 // coefficients (four of the thirteen operations of the 2D operator).
-template <class T, int RS>
+template <class T, int RS, bool CL>
 struct ResDiag {
     static constexpr bool kept = RS * sizeof(T) <= 16;
     T d[kept ? RS : 1][2];
-    __device__ __forceinline__ void load(const ResTile<T, RS>& t)
+    __device__ __forceinline__ void load(const ResTile<T, RS, CL>& t)
     {
         if constexpr (kept)
             t.sweep([&](int k, int q, const NbT<T>&, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
@@ -755,8 +995,8 @@ __device__ __forceinline__ void cg_note_pw(const FusedArgs& a, SolveState& s, do
 template <class P>
 __device__ __forceinline__ bool cg_after_rr(const FusedArgs& a, SolveState& s, double v)
 {
-    s.last_beta = v / s.rro;
-    s.rro = v;
+    // The loop test first: the division's call hides what is behind it from the scheduler.
+    const double rro = s.rro;
     if constexpr (P::fp32) {
         const int n = ++s.n_inner;
         const bool at_switch = s.switch_err > 0.0 && n >= s.switch_min && v <= s.switch_err;
@@ -765,6 +1005,8 @@ __device__ __forceinline__ bool cg_after_rr(const FusedArgs& a, SolveState& s, d
         s.error = v;
         end_iteration(a, s, PHASE_CG);
     }
+    s.rro = v;
+    s.last_beta = v / rro;
     return s.cont != 0;
 }
 template <class P>
@@ -785,18 +1027,19 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
 #define RES_PROLOGUE(P, RES_SCALE)                                                                 \
     using T = typename P::T;                                                                       \
     extern __shared__ __align__(16) unsigned char s_res_raw[];                                     \
-    __shared__ ResShared sh;                                                                       \
+    __shared__ ResShared<CL> sh;                                                                   \
     const FusedArgs& a = A.f;                                                                      \
     if (threadIdx.x == 0) {                                                                        \
         sh.s = A.start ? *A.start : A.s0;                                                          \
     }                                                                                              \
-    ResTile<T, RS> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                      \
+    ResTile<T, RS, CL> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                  \
     if (threadIdx.x == 0) t.start(RES_SCALE);                                                      \
-    ResDiag<T, RS> dg;                                                                             \
+    ResDiag<T, RS, CL> dg;                                                                             \
     SolveState& s = sh.s
 
 #define RES_EPILOGUE()                                                                             \
-    __syncthreads();                                                                               \
+    if constexpr (CL) res_cluster_sync(); /* nothing is on its way to a block that has ended */    \
+    else __syncthreads();                                                                          \
     if (blockIdx.x == 0) {                                                                         \
         if (threadIdx.x == 0) *a.st = *A.host = s;                                                 \
         t.clear_other_set();                                                                       \
@@ -805,7 +1048,7 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
 // CG: per iteration p = beta p + (z|r), w = A p and p.w; u += alpha p, r -= alpha w and
 // r.(r|z).  The neighbours' r arrives while the second sum is formed, and the halo of p follows
 // by the same recurrence, so an iteration waits for two sums and nothing else.
-template <class P, int RS, int W>
+template <class P, int RS, int W, bool CL>
 __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ ResArgs A)
 {
     RES_PROLOGUE(P, sh.s.rro);
@@ -814,7 +1057,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
     t.load_operand(P::p(a));
     if (pre) t.load_halo_mi(P::mi(a, pre));
     T r[RS][2], w[RS][2];
-    ResOwn<T, RS> u(t, P::u(a));
+    ResOwn<T, RS, CL> u(t, P::u(a));
 #pragma unroll
     for (int k = 0; k < RS; ++k) {
         r[k][0] = r[k][1] = w[k][0] = w[k][1] = (T)0;
@@ -822,9 +1065,17 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
     }
     __syncthreads();
     dg.load(t);
+    const int h0 = (int)threadIdx.x < t.nh ? t.table()[threadIdx.x].x : -1;
     for (bool pend = false;; pend = true) {
         if (pend) {
             const T beta = (T)s.last_beta;
+            // The thread's halo cell is loaded beside its own cells.
+            T hp = (T)0, hr = (T)0;
+            if (h0 >= 0) {
+                hp = t.V[h0];
+                hr = t.halo_r(threadIdx.x);
+                if (pre) hr = t.halo_mi(threadIdx.x) * hr;
+            }
 #pragma unroll
             for (int k = 0; k < RS; ++k)
                 if (t.on(k)) {
@@ -837,7 +1088,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
                     }
                     t.store(k, beta * c.x + q0, beta * c.y + q1);
                 }
-            for (int h = threadIdx.x; h < t.nh; h += blockDim.x) {
+            if (h0 >= 0) t.V[h0] = beta * hp + hr;
+            for (int h = threadIdx.x + blockDim.x; h < t.nh; h += blockDim.x) {
                 T q = t.halo_r(h);
                 if (pre) q = t.halo_mi(h) * q;
                 T* c = t.V + t.table()[h].x;
@@ -849,7 +1101,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
         t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
             const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
             w[k][q] = wv;
-            t.add(acc, q, (double)wv * (double)nb.c);
+            t.add(acc, k, q, (double)wv * (double)nb.c);
         });
         if (t.reduce(
                 acc, 0, [] {}, [&](double v) { return cg_after_pw(s, v); }, [&](double v) { cg_note_pw<P>(a, s, v); }) !=
@@ -857,7 +1109,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
             break;
         const T alpha = (T)s.alpha;
         acc.hi = acc.lo = 0.0;
-        ++t.tag;
+        t.next_exchange();
 #pragma unroll
         for (int k = 0; k < RS; ++k)
             if (t.on(k)) {
@@ -877,8 +1129,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
                     q0 = m.x * q0;
                     q1 = m.y * q1;
                 }
-                t.add(acc, 0, (double)r[k][0] * (double)q0);
-                t.add(acc, 1, (double)r[k][1] * (double)q1);
+                t.add(acc, k, 0, (double)r[k][0] * (double)q0);
+                t.add(acc, k, 1, (double)r[k][1] * (double)q1);
                 w[k][0] = w[k][0] + alpha * c.x;
                 w[k][1] = w[k][1] + alpha * c.y;
             }
@@ -914,7 +1166,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cg(const __grid_constant__ Re
 // Chebyshev: r = rhs - A u, p = alpha p + beta (mi r | r), u += p.  Iterations between two
 // checks only exchange the rim of u with the neighbouring tiles; r.r is summed where the loop
 // checks it.
-template <class P, int RS, int W>
+template <class P, int RS, int W, bool CL>
 __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__ ResArgs A)
 {
     RES_PROLOGUE(P, P::fp32 ? sh.s.rro : sh.s.error);
@@ -922,7 +1174,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
     t.load_coefs(P::kx(a), P::ky(a), P::kz(a), P::mi(a, pre));
     t.load_operand(P::u(a));
     T p[RS][2], un[RS][2];
-    const ResOwn<T, RS> b(t, P::rhs(a));
+    const ResOwn<T, RS, CL> b(t, P::rhs(a));
 #pragma unroll
     for (int k = 0; k < RS; ++k) {
         p[k][0] = p[k][1] = un[k][0] = un[k][1] = (T)0;
@@ -935,7 +1187,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
         const T al = (T)a.ch_alphas[step], be = (T)a.ch_betas[step];
         const bool check = P::fp32 ? s.n_inner % 10 == 0 : (s.n >= s.est_itc && s.n % 10 == 0);
         DD acc = {0.0, 0.0};
-        ++t.tag;
+        t.next_exchange();
         Two<T> m;
         m.x = m.y = (T)1;
         b.load(t, un);
@@ -946,7 +1198,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
             const T pv = al * p[k][q] + be * (pre ? (q == 0 ? m.x : m.y) * rv : rv);
             p[k][q] = pv;
             un[k][q] = nb.c + pv;
-            if (check) t.add(acc, q, (double)rv * (double)rv);
+            if (check) t.add(acc, k, q, (double)rv * (double)rv);
         });
 #pragma unroll
         for (int k = 0; k < RS; ++k)
@@ -988,7 +1240,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
 
 // PPCG without the preconditioner: the CG sweep on p, then the inner steps on sd, each with
 // one rim exchange; V holds p and then sd.
-template <class P, int RS, int W>
+template <class P, int RS, int W, bool CL>
 __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ ResArgs A)
 {
     RES_PROLOGUE(P, sh.s.rro);
@@ -996,7 +1248,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
     t.load_operand(P::p(a));
     constexpr bool PREG = RS * sizeof(T) <= 16;  // p waits in registers, else in its array, for the next outer iteration
     T r[RS][2], w[RS][2], p[PREG ? RS : 1][2];
-    ResOwn<T, RS> u(t, P::u(a));
+    ResOwn<T, RS, CL> u(t, P::u(a));
 #pragma unroll
     for (int k = 0; k < RS; ++k) {
         r[k][0] = r[k][1] = w[k][0] = w[k][1] = (T)0;
@@ -1020,7 +1272,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
     for (bool pend = false;; pend = true) {
         if (pend) {
             const T beta = (T)s.last_beta;
-            ++t.tag;
+            t.next_exchange();
             if constexpr (PREG) {
 #pragma unroll
                 for (int k = 0; k < RS; ++k) {
@@ -1051,7 +1303,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
         t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
             const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
             w[k][q] = wv;
-            t.add(acc, q, (double)wv * (double)nb.c);
+            t.add(acc, k, q, (double)wv * (double)nb.c);
         });
         if (t.reduce(
                 acc, 0, [] {}, [&](double v) { return cg_after_pw(s, v); },
@@ -1062,7 +1314,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                 }) != RN_GO)
             break;
         const T alpha = (T)s.alpha, theta = (T)s.theta;
-        ++t.tag;
+        t.next_exchange();
 #pragma unroll
         for (int k = 0; k < RS; ++k)
             if (t.on(k)) {
@@ -1100,11 +1352,11 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                 const T rv = r[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
                 r[k][q] = rv;
                 w[k][q] = al * nb.c + be * rv;
-                if (last) t.add(acc, q, (double)rv * (double)rv);
+                if (last) t.add(acc, k, q, (double)rv * (double)rv);
             });
             if (last) break;
             __syncthreads();  // every warp has read the old sd
-            ++t.tag;
+            t.next_exchange();
 #pragma unroll
             for (int k = 0; k < RS; ++k)
                 if (t.on(k)) set_operand(k, w[k][0], w[k][1]);
@@ -1155,14 +1407,14 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
 
 // Jacobi: u_new = (rhs + sum K u) / diagonal and sum |u_new - u|; every 50th iteration the
 // true residual instead.
-template <class P, int RS, int W>
+template <class P, int RS, int W, bool CL>
 __global__ void __launch_bounds__(32 * W, 1) k_res_jacobi(const __grid_constant__ ResArgs A)
 {
     RES_PROLOGUE(P, sh.s.error);
     t.load_coefs(a.kx, a.ky, a.kz, nullptr);
     t.load_operand(a.u[0]);
     T un[RS][2];
-    const ResOwn<T, RS> b(t, a.u0);
+    const ResOwn<T, RS, CL> b(t, a.u0);
 #pragma unroll
     for (int k = 0; k < RS; ++k) un[k][0] = un[k][1] = (T)0;
     __syncthreads();
@@ -1170,12 +1422,12 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_jacobi(const __grid_constant_
     for (;;) {
         const bool residual = s.n % 50 == 0;
         DD acc = {0.0, 0.0};
-        ++t.tag;
+        t.next_exchange();
         b.load(t, un);
         t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
             const T v = jacobi_k(un[k][q], nb, kx0, kx1, ky0, ky1, kz0, kz1);
             un[k][q] = v;
-            t.add(acc, q, fabs(v - nb.c));
+            t.add(acc, k, q, fabs(v - nb.c));
         });
 #pragma unroll
         for (int k = 0; k < RS; ++k)
@@ -1198,7 +1450,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_jacobi(const __grid_constant_
             b.load(t, un);
             t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
                 un[k][q] = un[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
-                t.add(acc, q, un[k][q] * un[k][q]);
+                t.add(acc, k, q, un[k][q] * un[k][q]);
             });
 #pragma unroll
             for (int k = 0; k < RS; ++k)

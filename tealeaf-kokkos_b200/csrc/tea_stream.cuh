@@ -472,10 +472,10 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_con
 {
     using T = typename P::T;
     extern __shared__ __align__(16) unsigned char s_stream_raw[];
-    __shared__ ResShared sh;
+    __shared__ ResShared<false> sh;
     const FusedArgs& a = A.f;
     SolveState& s = sh.s;
-    GridSum sum(A.sum, sh.sum);
+    GridSum<> sum(A.sum, sh.sum);
     if (threadIdx.x == 0) {
         s = A.start ? *A.start : A.s0;
         sum.start(s.rro);

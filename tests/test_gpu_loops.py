@@ -21,6 +21,9 @@ FIELDS = ("iterations", "error", "exact_error", "vol", "mass", "ie", "temp")
 STREAM_SHAPES = {2: [(1101, 1003), (4099, 300), (300, 4100)], 3: [(101, 99, 97), (3, 200, 100), (257, 66, 65)]}
 SHAPES = {2: [(7, 5), (65, 16), (64, 17), (131, 33), (700, 37), (257, 515), (701, 699), (860, 850), (1023, 1009)],
           3: [(5, 4, 3), (65, 9, 8), (31, 30, 29), (48, 48, 48), (66, 52, 77), (80, 77, 76)]}
+# One cluster: cut along each axis and along two, into few blocks and into sixteen, odd tiles.
+CLUSTER_SHAPES = {2: [(2, 33), (129, 11), (131, 35), (33, 150), (127, 128)],
+                  3: [(17, 7, 9), (33, 16, 5), (66, 5, 24), (30, 2, 61), (63, 15, 16)]}
 
 
 def _deck(dim, shape, solver, precond):
@@ -67,6 +70,13 @@ def test_on_chip_loops_equal_per_call(dim, shape, solver, precond):
     _same(_run(deck, dim, fused=True), _run(deck, dim))
 
 
+@pytest.mark.parametrize("solver,precond", [("cg", True), ("chebyshev", False), ("ppcg", False), ("jacobi", False)])
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in CLUSTER_SHAPES[d]])
+def test_cluster_loops_equal_per_call(dim, shape, solver, precond):
+    deck = _deck(dim, shape, solver, precond)
+    _same(_run(deck, dim, fused=True), _run(deck, dim))
+
+
 @pytest.mark.parametrize("precond", [False, True])
 @pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in STREAM_SHAPES[d]])
 def test_streaming_cg_equals_per_call(dim, shape, precond):
@@ -75,7 +85,7 @@ def test_streaming_cg_equals_per_call(dim, shape, precond):
 
 
 @pytest.mark.parametrize("solver", ["cg", "chebyshev", "ppcg"])
-@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2] + STREAM_SHAPES[d][::2]])
+@pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in SHAPES[d][1::2] + CLUSTER_SHAPES[d][::2] + STREAM_SHAPES[d][::2]])
 def test_one_launch_fp32_loops_equal_single_launches(dim, shape, solver):
     deck = _deck(dim, shape, solver, False)
     kw = {"fused": True, "precision": tea.PRECISION_FP32_REFINED}

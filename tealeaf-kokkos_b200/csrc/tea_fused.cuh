@@ -128,6 +128,30 @@ __device__ __forceinline__ T smvp_k(const NbT<T>& a, T kx0, T kx1, T ky0, T ky1,
 #endif
 }
 
+// The operator's diagonal at a cell, and the operator with it given: smvp_k()'s expression.
+template <class T>
+__device__ __forceinline__ T diag_k(T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
+{
+#if TEA_DIM == 2
+    (void)kz0;
+    (void)kz1;
+    return (T)1 + (kx1 + kx0) + (ky1 + ky0);
+#else
+    return (T)1 + (kx1 + kx0) + (ky1 + ky0) + (kz1 + kz0);
+#endif
+}
+template <class T>
+__device__ __forceinline__ T smvp_dk(T d, const NbT<T>& a, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
+{
+#if TEA_DIM == 2
+    (void)kz0;
+    (void)kz1;
+    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym);
+#else
+    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym) - (kz1 * a.zp + kz0 * a.zm);
+#endif
+}
+
 __device__ __forceinline__ double jacobi_k(double u0, const Nb& a, double kx0, double kx1, double ky0, double ky1,
                                            double kz0, double kz1)
 {
@@ -1439,6 +1463,13 @@ struct PpcgF32 {
 // (x-neighbours come by shuffle), and the preconditioner's rows only in the PRE form: without
 // them a slot of TY = 8 is 51 rows of 512 bytes, so that with one plane in flight (RP = 1)
 // two blocks fit on an SM.
+//
+// What bounds it: the issue slots and latencies of the 16 warps that registers and shared memory
+// allow on an SM (256^3: DRAM at 51 % of its peak, issue slots 56 % busy; more rows a tile in one
+// block, which does less twice, is slower: 16 rows 319 us against 306).  So the work per plane was
+// cut: Kz and the operator's diagonal are carried from plane to plane and from step k to step k+1
+// in registers, and the plane loop is unrolled by the length of the register rotations.  Two steps at
+// 256^3: 306 -> 291 us, with the preconditioner 420 -> 371, FP32 220 -> 210; 131x97x200: 80 -> 74.
 template <int TY, bool PRE>
 struct Ppcg2Rows {
     static constexpr int RAW = 0;                      // sd: TY + 2 rows
@@ -1459,7 +1490,7 @@ constexpr size_t ppcg2_smem_bytes()
 }
 
 template <class P, int TY, int RP, bool PRE>
-__global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
+__global__ void __launch_bounds__(TY * 32, PRE ? 1 : 2) k_ppcg2_ring3d(FusedArgs a)
 {
     using T = typename P::T;
     extern __shared__ __align__(16) unsigned char s_raw[];
@@ -1521,7 +1552,7 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
         const int r_below = refl(y0 - 1, g.Y);
         const int r_above = refl(min(y0 + TY, ylast + 1), g.Y);
         const int i_above = min(y0 + TY, ylast + 1);
-        auto slot = [&](int p) { return ring + (size_t)((p - zf + 1) % RQ) * SLOT; };
+        auto slot = [&](int p) { return ring + (unsigned)(p - zf + 1) % RQ * SLOT; };
         // Plane p of the tile: sd at the warps' rows for planes zf-1 .. zl+1, the rest for
         // step k's planes, Kz also for plane zl+1.
         auto issue = [&](int p) {
@@ -1547,21 +1578,20 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
         };
         auto own = [&](const T* base, int row, T* v) { ld_vec(base + row * RWT + OFF + VEC * lane, v); };
         // Step k at plane p from sd at planes p-1 (A), p (B), p+1 (C): r1, u1 and sd1 at the
-        // lane's cells; sd1 also into the shared plane buffer.
-        auto step1 = [&](int p, const T* A, const T* B, const T* C, T* r1, T* u1, T* t1) {
+        // lane's cells, and the operator's diagonal d1 there; sd1 also into the shared plane
+        // buffer.  kz0, kz1: the lower faces' coefficients of planes p and p+1.
+        auto step1 = [&](int p, const T* A, const T* B, const T* C, const T* kz0, const T* kz1, T* r1, T* u1, T* t1,
+                         T* d1) {
             const T* cur = slot(p);
-            const T* nxt = slot(p + 1);
             const T up = __shfl_up_sync(0xffffffffu, B[VEC - 1], 1);
             const T dn = __shfl_down_sync(0xffffffffu, B[0], 1);
             T kx[VEC + 1];
             own(cur, R::KX + w, kx);
             kx[VEC] = __shfl_down_sync(0xffffffffu, kx[0], 1);
             if (p <= zl && row_in) {
-                T ky0[VEC], ky1[VEC], kz0[VEC], kz1[VEC], ym[VEC], yp[VEC], rr[VEC], uu[VEC], mi[VEC];
+                T ky0[VEC], ky1[VEC], ym[VEC], yp[VEC], rr[VEC], uu[VEC], mi[VEC];
                 own(cur, R::KY + w, ky0);
                 own(cur, R::KY + w + 1, ky1);
-                own(cur, R::KZ + w, kz0);
-                own(nxt, R::KZ + w, kz1);
                 own(cur, R::RAW + w, ym);
                 own(cur, R::RAW + w + 2, yp);
                 own(cur, IN_R + w, rr);
@@ -1571,13 +1601,14 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
                 for (int q = 0; q < VEC; ++q) {
                     NbT<T> nb;
                     nb.c = B[q];
-                    nb.xm = c + q == HALO_PAD ? B[q] : (q == 0 ? up : B[q > 0 ? q - 1 : 0]);
+                    nb.xm = q > 0 ? B[q > 0 ? q - 1 : 0] : (c == HALO_PAD ? B[q] : up);  // c is HALO_PAD plus a multiple of VEC
                     nb.xp = c + q == xlast ? B[q] : (q == VEC - 1 ? dn : B[q < VEC - 1 ? q + 1 : q]);
                     nb.ym = ym[q];
                     nb.yp = yp[q];
                     nb.zm = A[q];
                     nb.zp = C[q];
-                    const T s = smvp_k(nb, kx[q], kx[q + 1], ky0[q], ky1[q], kz0[q], kz1[q]);
+                    d1[q] = diag_k(kx[q], kx[q + 1], ky0[q], ky1[q], kz0[q], kz1[q]);
+                    const T s = smvp_dk(d1[q], nb, kx[q], kx[q + 1], ky0[q], ky1[q], kz0[q], kz1[q]);
                     const T r = rr[q] - s;
                     r1[q] = r;
                     u1[q] = uu[q] + B[q];
@@ -1585,7 +1616,7 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
                 }
             } else {
 #pragma unroll
-                for (int q = 0; q < VEC; ++q) r1[q] = u1[q] = t1[q] = (T)0;
+                for (int q = 0; q < VEC; ++q) r1[q] = u1[q] = t1[q] = d1[q] = (T)0;
             }
             st_vec(s1 + ((size_t)(p & 1) * TY + w) * STRIP + VEC * lane, t1);
         };
@@ -1595,36 +1626,41 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
         T sA[VEC], sB[VEC], sC[VEC];  // sd at planes z, z+1, z+2 (the warp's row)
         T tm[VEC], tc[VEC], tn[VEC];  // step k's sd at planes z-1, z, z+1
         T r1c[VEC], u1c[VEC], r1n[VEC], u1n[VEC];
+        // Kz of planes z, z+1, z+2 and the diagonal of planes z, z+1, carried along: read and formed
+        // once for both steps.
+        T kzA[VEC], kzB[VEC], kzC[VEC], dc[VEC], dn1[VEC];
         {
             T sM[VEC];
             own(slot(zf - 1), R::RAW + w + 1, sM);
             own(slot(zf), R::RAW + w + 1, sA);
             own(slot(zf + 1), R::RAW + w + 1, sB);
-            step1(zf, sM, sA, sB, r1c, u1c, tc);
+            own(slot(zf), R::KZ + w, kzA);
+            own(slot(zf + 1), R::KZ + w, kzB);
+            step1(zf, sM, sA, sB, kzA, kzB, r1c, u1c, tc, dc);
 #pragma unroll
             for (int q = 0; q < VEC; ++q) tm[q] = tc[q];
         }
+        // By three: the planes' values then rotate through the registers without moves.
+#pragma unroll 3
         for (int z = zf; z < z1; ++z) {
             cp_async_wait<RP - 1>();
             __syncthreads();
             issue(z + RP + 2);  // into the slot of plane z - 1, which no warp reads any more
             own(slot(z + 2), R::RAW + w + 1, sC);
-            step1(z + 1, sA, sB, sC, r1n, u1n, tn);
+            own(slot(z + 2), R::KZ + w, kzC);
+            step1(z + 1, sA, sB, sC, kzB, kzC, r1n, u1n, tn, dn1);
             if (z >= z0) {
                 // Step k+1 at plane z.
                 const T* cur = slot(z);
-                const T* nxt = slot(z + 1);
                 const T up = __shfl_up_sync(0xffffffffu, tc[VEC - 1], 1);
                 const T dn = __shfl_down_sync(0xffffffffu, tc[0], 1);
                 T kx[VEC + 1];
                 own(cur, R::KX + w, kx);
                 kx[VEC] = __shfl_down_sync(0xffffffffu, kx[0], 1);
                 if (row_out && lane_out) {
-                    T ky0[VEC], ky1[VEC], kz0[VEC], kz1[VEC], ym[VEC], yp[VEC], mi[VEC];
+                    T ky0[VEC], ky1[VEC], ym[VEC], yp[VEC], mi[VEC];
                     own(cur, R::KY + w, ky0);
                     own(cur, R::KY + w + 1, ky1);
-                    own(cur, R::KZ + w, kz0);
-                    own(nxt, R::KZ + w, kz1);
                     if (precond) own(cur, IN_MI + w, mi);
                     const T* sp = s1 + (size_t)(z & 1) * TY * STRIP + VEC * lane;
                     if (j > HALO_PAD) ld_vec(sp + (w - 1) * STRIP, ym);
@@ -1634,13 +1670,13 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
                     for (int q = 0; q < VEC; ++q) {
                         NbT<T> nb;
                         nb.c = tc[q];
-                        nb.xm = c + q == HALO_PAD ? tc[q] : (q == 0 ? up : tc[q > 0 ? q - 1 : 0]);
+                        nb.xm = q > 0 ? tc[q > 0 ? q - 1 : 0] : (c == HALO_PAD ? tc[q] : up);
                         nb.xp = c + q == xlast ? tc[q] : (q == VEC - 1 ? dn : tc[q < VEC - 1 ? q + 1 : q]);
                         nb.ym = j == HALO_PAD ? tc[q] : ym[q];
                         nb.yp = j == ylast ? tc[q] : yp[q];
                         nb.zm = z == HALO_PAD ? tc[q] : tm[q];
                         nb.zp = z == zlast ? tc[q] : tn[q];
-                        const T s = smvp_k(nb, kx[q], kx[q + 1], ky0[q], ky1[q], kz0[q], kz1[q]);
+                        const T s = smvp_dk(dc[q], nb, kx[q], kx[q + 1], ky0[q], ky1[q], kzA[q], kzB[q]);
                         const T r = r1c[q] - s;
                         r2[q] = r;
                         u2[q] = u1c[q] + tc[q];
@@ -1672,6 +1708,9 @@ __global__ void __launch_bounds__(TY * 32) k_ppcg2_ring3d(FusedArgs a)
                 tc[q] = tn[q];
                 r1c[q] = r1n[q];
                 u1c[q] = u1n[q];
+                kzA[q] = kzB[q];
+                kzB[q] = kzC[q];
+                dc[q] = dn1[q];
             }
         }
         cp_async_wait<0>();

@@ -933,30 +933,6 @@ struct ResOwn {
     }
 };
 
-// The operator's diagonal at a cell, and the operator with it given: smvp_k's expression.
-template <class T>
-__device__ __forceinline__ T res_diag(T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
-{
-#if TEA_DIM == 2
-    (void)kz0;
-    (void)kz1;
-    return (T)1 + (kx1 + kx0) + (ky1 + ky0);
-#else
-    return (T)1 + (kx1 + kx0) + (ky1 + ky0) + (kz1 + kz0);
-#endif
-}
-template <class T>
-__device__ __forceinline__ T res_smvp(T d, const NbT<T>& a, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1)
-{
-#if TEA_DIM == 2
-    (void)kz0;
-    (void)kz1;
-    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym);
-#else
-    return d * a.c - (kx1 * a.xp + kx0 * a.xm) - (ky1 * a.yp + ky0 * a.ym) - (kz1 * a.zp + kz0 * a.zm);
-#endif
-}
-
 // Diagonals of the warp's cells: in registers where there is room, else formed again from the
 // coefficients (four of the thirteen operations of the 2D operator).
 template <class T, int RS, bool CL>
@@ -967,12 +943,12 @@ struct ResDiag {
     {
         if constexpr (kept)
             t.sweep([&](int k, int q, const NbT<T>&, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
-                d[k][q] = res_diag(kx0, kx1, ky0, ky1, kz0, kz1);
+                d[k][q] = diag_k(kx0, kx1, ky0, ky1, kz0, kz1);
             });
     }
     __device__ __forceinline__ T smvp(int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) const
     {
-        if constexpr (kept) return res_smvp(d[k][q], nb, kx0, kx1, ky0, ky1, kz0, kz1);
+        if constexpr (kept) return smvp_dk(d[k][q], nb, kx0, kx1, ky0, ky1, kz0, kz1);
         else return smvp_k(nb, kx0, kx1, ky0, ky1, kz0, kz1);
     }
 };

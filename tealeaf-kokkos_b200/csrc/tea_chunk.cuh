@@ -76,7 +76,7 @@ struct Chunk {
     RedScratch red{};
     double* h_out = nullptr;  // mapped pinned host memory for reduction results
     double* d_out = nullptr;  // its device alias
-    volatile unsigned int* h_done = nullptr;  // mapped, behind the results: the ticket of the last one
+    volatile unsigned long long* h_post = nullptr;  // mapped, behind the results: the posted ones' word pairs
     int grid_blocks = 0;      // blocks for grid-stride per-call kernels
     int device = 0;
     void* fused = nullptr;    // whole-solve state (tea_fused.cuh)

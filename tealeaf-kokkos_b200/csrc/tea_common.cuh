@@ -91,9 +91,22 @@ struct RedScratch {
     DD* partials;           // [max_blocks * MAX_RED]
     unsigned int* counter;  // reset to 0 by the last block
     int max_blocks;
-    unsigned int* done;     // host memory: takes `ticket` once a result is in host memory (null: none)
-    unsigned int ticket;
+    unsigned long long* done;   // host memory: takes a word pair per result under `ticket` (null: none)
+    unsigned long long ticket;
 };
+
+// A result for a host that polls: the value's bits and, in the same 16-byte store, a word that says
+// which launch they belong to.  No fence orders anything: a pair of which the host sees only one half
+// does not pass posted().
+__host__ __device__ inline unsigned long long post_check(unsigned long long bits, unsigned long long ticket)
+{
+    return bits ^ (ticket * 0x9E3779B97F4A7C15ull);
+}
+__device__ __forceinline__ void post_result(unsigned long long* to, double v, unsigned long long ticket)
+{
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+    asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(to), "l"(bits), "l"(post_check(bits, ticket)) : "memory");
+}
 
 template <int NV>
 __device__ __forceinline__ void warp_merge(DDVec<NV>& a)
@@ -110,18 +123,70 @@ __device__ __forceinline__ void warp_merge(DDVec<NV>& a)
     }
 }
 
-// Last block of a grid reduction: every thread merges a strided share of the block
-// partials (up to four loads in flight per thread), then a fixed-order warp merge and a
-// merge of the warps in order through `s` (nwarps x NV, shared).  The order depends only on
-// the grid and block sizes.  Called by every thread of the last block; the result is valid
-// in thread 0.
+// Merge over a block: butterflies in the warps, then over the warps' values in warp 0, through `s`
+// (nwarps x NV, shared).  Called by every thread; the result is valid in warp 0.
 template <int NV>
-__device__ __forceinline__ DDVec<NV> merge_partials(const RedScratch& rs, DD* s, int tid, int nthreads)
+__device__ __forceinline__ DDVec<NV> block_merge(DDVec<NV> a, DD* s, int tid, int nwarps)
 {
-    const int lane = tid & 31, warp = tid >> 5, nwarps = nthreads >> 5;
-    DDVec<NV> b;
-    b.zero();
+    const int lane = tid & 31, warp = tid >> 5;
+    warp_merge<NV>(a);
+    if (nwarps == 1) return a;
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) s[warp * NV + k] = a.v[k];
+    }
+    __syncthreads();
+    if (warp == 0) {
+        a.zero();
+        if (lane < nwarps) {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) a.v[k] = s[lane * NV + k];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            if (o >= nwarps) continue;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                DD b;
+                b.hi = __shfl_xor_sync(0xffffffffu, a.v[k].hi, o);
+                b.lo = __shfl_xor_sync(0xffffffffu, a.v[k].lo, o);
+                a.v[k] = dd_merge(a.v[k], b);
+            }
+        }
+    }
+    return a;
+}
+
+// The sum over the grid, valid in thread 0 of the block for which `last` comes back true (the last
+// to arrive, which merges the blocks' partials).  The order depends only on the grid and block
+// sizes; no block waits on another.  Called by every thread of the block.
+//
+// At the per-call kernels' sizes this tail is latency from end to end: with serial merges by one
+// thread (the warps' values, twice), a fence on either side of the arrival and one more before the
+// host's word a reduction took 2 us longer (ext_cg_calc_w_, call to result: 14.5 us on 10 x 10
+// cells and 14.8 at 512 x 512, now 12.6 and 12.7).
+template <int NV>
+__device__ __forceinline__ DDVec<NV> grid_merge(const DDVec<NV>& acc, const RedScratch& rs, DD* s, int tid, int nwarps,
+                                                bool& last)
+{
+    __shared__ bool s_last;
+    DDVec<NV> b = block_merge<NV>(acc, s, tid, nwarps);
     const int nblk = (int)gridDim.x;
+    last = true;
+    if (nblk == 1) return b;
+    if (tid == 0) {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) rs.partials[(long)blockIdx.x * MAX_RED + k] = b.v[k];
+        unsigned int prev;
+        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(rs.counter) : "memory");
+        s_last = prev == (unsigned)nblk - 1;
+    }
+    __syncthreads();
+    last = s_last;
+    if (!last) return b;
+    // Every thread merges a strided share of the partials, four loads in flight.
+    const int nthreads = nwarps * 32;
+    b.zero();
     for (int blk0 = tid; blk0 < nblk; blk0 += 4 * nthreads) {
         DD p[4][NV];
 #pragma unroll
@@ -134,68 +199,30 @@ __device__ __forceinline__ DDVec<NV> merge_partials(const RedScratch& rs, DD* s,
             }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < 4; ++u) {
+            if (u > 0 && blk0 + u * nthreads >= nblk) break;
 #pragma unroll
             for (int k = 0; k < NV; ++k) b.v[k] = dd_merge(b.v[k], p[u][k]);
+        }
     }
-    warp_merge<NV>(b);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) s[warp * NV + k] = b.v[k];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        b.zero();
-        for (int w = 0; w < nwarps; ++w)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) b.v[k] = dd_merge(b.v[k], s[w * NV + k]);
-    }
-    return b;
+    if (tid == 0) *rs.counter = 0u;
+    return block_merge<NV>(b, s, tid, nwarps);
 }
 
-// Block-reduce `acc`, then the last block to arrive merges every block's partial in
-// block order and writes the rounded results to out[0..NV).  Deterministic for a given
-// grid size; no block waits on another.  Must be called by every thread of the block.
+// Reduce over the grid; the last block writes the rounded results to out[0..NV), or posts them to
+// the host where it waits for them.  Must be called by every thread of the block.
 template <int NV>
 __device__ void grid_reduce(DDVec<NV> acc, const RedScratch& rs, double* out)
 {
     __shared__ DD s_warp[BLOCK / 32][NV];
-    __shared__ bool s_last;
-    const int lane = threadIdx.x & 31;
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-    const int warp = tid >> 5;
-    const int nwarps = (blockDim.x * blockDim.y) >> 5;
-    warp_merge<NV>(acc);
-    if (lane == 0) {
+    bool last;
+    const DDVec<NV> b = grid_merge<NV>(acc, rs, &s_warp[0][0], tid, (blockDim.x * blockDim.y) >> 5, last);
+    if (last && tid == 0) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) s_warp[warp][k] = acc.v[k];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        DDVec<NV> b;
-        b.zero();
-        for (int w = 0; w < nwarps; ++w)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) b.v[k] = dd_merge(b.v[k], s_warp[w][k]);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) rs.partials[(long)blockIdx.x * MAX_RED + k] = b.v[k];
-        __threadfence();
-        const unsigned int prev = atomicAdd(rs.counter, 1u);
-        s_last = (prev == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last) return;
-    // Last block: every thread merges a share of the partials (fixed order).
-    __threadfence();
-    const DDVec<NV> b = merge_partials<NV>(rs, &s_warp[0][0], tid, nwarps * 32);
-    if (tid == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) out[k] = dd_value(b.v[k]);
-        *rs.counter = 0u;
-        if (rs.done) {
-            // Every other block has ended its work: the host need not wait for the launch to retire.
-            __threadfence_system();
-            *(volatile unsigned int*)rs.done = rs.ticket;
+        for (int k = 0; k < NV; ++k) {
+            if (rs.done) post_result(rs.done + 2 * k, dd_value(b.v[k]), rs.ticket);
+            else out[k] = dd_value(b.v[k]);
         }
     }
 }
@@ -206,38 +233,13 @@ template <int NV, class F>
 __device__ void grid_reduce_then(DDVec<NV> acc, const RedScratch& rs, F&& f)
 {
     __shared__ DD s_warp2[32][NV];
-    __shared__ bool s_last2;
-    const int lane = threadIdx.x & 31;
     const int tid = threadIdx.x + threadIdx.y * blockDim.x;
-    const int warp = tid >> 5;
-    const int nwarps = (blockDim.x * blockDim.y) >> 5;
-    warp_merge<NV>(acc);
-    if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) s_warp2[warp][k] = acc.v[k];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        DDVec<NV> b;
-        b.zero();
-        for (int w = 0; w < nwarps; ++w)
-#pragma unroll
-            for (int k = 0; k < NV; ++k) b.v[k] = dd_merge(b.v[k], s_warp2[w][k]);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) rs.partials[(long)blockIdx.x * MAX_RED + k] = b.v[k];
-        __threadfence();
-        const unsigned int prev = atomicAdd(rs.counter, 1u);
-        s_last2 = (prev == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!s_last2) return;
-    __threadfence();
-    const DDVec<NV> b = merge_partials<NV>(rs, &s_warp2[0][0], tid, nwarps * 32);
-    if (tid == 0) {
+    bool last;
+    const DDVec<NV> b = grid_merge<NV>(acc, rs, &s_warp2[0][0], tid, (blockDim.x * blockDim.y) >> 5, last);
+    if (last && tid == 0) {
         double vals[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) vals[k] = dd_value(b.v[k]);
-        *rs.counter = 0u;
         f(vals);
     }
 }

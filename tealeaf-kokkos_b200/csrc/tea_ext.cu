@@ -147,12 +147,12 @@ Chunk* create_chunk(int nx, int ny, int nz, int rank)
     TEA_CK(cudaMalloc(&c->red.partials, sizeof(DD) * MAX_RED * c->red.max_blocks));
     TEA_CK(cudaMalloc(&c->red.counter, sizeof(unsigned int)));
     TEA_CK(cudaMemset(c->red.counter, 0, sizeof(unsigned int)));
-    // Eight results and, on a cache line of its own, the ticket of the last one.
+    // Eight results and, on a cache line of their own, the word pairs of four posted ones.
     TEA_CK(cudaHostAlloc(&c->h_out, 16 * sizeof(double), cudaHostAllocMapped));
     TEA_CK(cudaHostGetDevicePointer(&c->d_out, c->h_out, 0));
     if (c->h_out) {
         std::memset(c->h_out, 0, 16 * sizeof(double));
-        c->h_done = reinterpret_cast<volatile unsigned int*>(c->h_out + 8);
+        c->h_post = reinterpret_cast<volatile unsigned long long*>(c->h_out + 8);
     }
     c->red.done = nullptr;
     c->red.ticket = 0;
@@ -188,32 +188,41 @@ RedScratch awaited(Chunk* c)
 {
     ++c->red.ticket;
     RedScratch rs = c->red;
-    rs.done = c->h_done ? reinterpret_cast<unsigned int*>(c->d_out + 8) : nullptr;
+    rs.done = c->h_post ? reinterpret_cast<unsigned long long*>(c->d_out + 8) : nullptr;
     return rs;
 }
 
-// Waits for the results of the launch that got the last ticket.  The last block writes them and
-// then the ticket to host memory, which the host sees some 6 us before a stream synchronisation
-// would return; results that take longer than the spin, and launches that failed, are waited for
-// by a synchronisation, which also reports the error.
-void await_result(Chunk* c)
+// Whether result k of the launch that got the last ticket has arrived; then it is in h_out.
+static bool posted(Chunk* c, int k)
 {
-    TEA_CK(cudaGetLastError());
-    const unsigned int want = c->red.ticket;
-    const auto start = std::chrono::steady_clock::now();
-    while (c->h_done && *c->h_done != want) {
-        for (int k = 0; k < 64 && *c->h_done != want; ++k) {
-        }
-        if (std::chrono::steady_clock::now() - start > std::chrono::microseconds(500)) break;
-    }
-    std::atomic_thread_fence(std::memory_order_acquire);
-    if (!c->h_done || *c->h_done != want) sync(c);
+    const unsigned long long bits = c->h_post[2 * k], check = c->h_post[2 * k + 1];
+    if (check != post_check(bits, c->red.ticket)) return false;
+    std::memcpy(&c->h_out[k], &bits, sizeof(double));
+    return true;
 }
 
-// Result of a reduction kernel written through the mapped pointer.
+// Waits for the n results of the launch that got the last ticket.  The last block posts them to
+// host memory, which the host sees some 6 us before a stream synchronisation would return;
+// results that take longer than the spin, and launches that failed, are waited for by a
+// synchronisation, which also reports the error.
+void await_result(Chunk* c, int n)
+{
+    TEA_CK(cudaGetLastError());
+    const auto start = std::chrono::steady_clock::now();
+    int k = 0;
+    for (int spin = 1; c->h_post && k < n; ++spin) {
+        if (posted(c, k)) ++k;
+        else if (spin % 64 == 0 && std::chrono::steady_clock::now() - start > std::chrono::microseconds(500)) break;
+    }
+    if (k == n) return;
+    sync(c);
+    for (; c->h_post && k < n; ++k) posted(c, k);
+}
+
+// Result of a reduction kernel.
 double result(Chunk* c, int k)
 {
-    await_result(c);
+    await_result(c, k + 1);
     c->d2h_bytes += sizeof(double);
     return ((volatile double*)c->h_out)[k];
 }
@@ -461,7 +470,7 @@ TEA_EXPORT void ext_field_summary_kernel_(const int* chunk, double* vol, double*
     if (!c) return;
     k_field_summary<<<launch_blocks(c, c->inner.ntiles), dim3(TILE_X, TILE_Y), 0, c->stream>>>(
         c->g, c->inner, c->f, awaited(c), c->d_out);
-    await_result(c);
+    await_result(c, 4);
     c->d2h_bytes += 4 * sizeof(double);
     volatile double* h = c->h_out;
     *vol = h[0];

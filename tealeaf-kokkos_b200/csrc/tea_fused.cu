@@ -462,7 +462,7 @@ ResPlan res_plan(const Geom& g, int sms, int cluster, int elem, bool pre, size_t
                     }
                     const double wait = p.blocks == 1 ? 0.0 : (cl ? 500.0 + 10.0 * p.blocks : 1200.0 + 4.0 * p.blocks);
                     const double cost =
-                        (form + 1 == RES_FORM_COUNT ? 900.0 : 450.0) * rows * (0.4 + 0.6 * p.warps / RES_WARPS) + wait +
+                        (RES_FORMS[form].rows > 4 && warps > 12 ? 900.0 : 450.0) * rows * (0.4 + 0.6 * p.warps / RES_WARPS) + wait +
                         (p.blocks > 1 ? 150.0 * p.halo / (32.0 * p.warps) : 0.0);
                     if (best.blocks == 0 || cost < best_cost) {
                         best = p;
@@ -577,14 +577,15 @@ const void* res_kernel(int kind)
 template <class P>
 const void* res_kernel(int kind, int form)
 {
-    static_assert(RES_FORM_COUNT == 6, "every form has its kernels");
+    static_assert(RES_FORM_COUNT == 7, "every form has its kernels");
     switch (form) {
     case 0: return res_kernel<P, 0>(kind);
     case 1: return res_kernel<P, 1>(kind);
     case 2: return res_kernel<P, 2>(kind);
     case 3: return res_kernel<P, 3>(kind);
     case 4: return res_kernel<P, 4>(kind);
-    default: return res_kernel<P, 5>(kind);
+    case 5: return res_kernel<P, 5>(kind);
+    default: return res_kernel<P, 6>(kind);
     }
 }
 

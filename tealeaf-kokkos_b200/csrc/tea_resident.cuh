@@ -14,9 +14,9 @@
 // Work split.  A warp owns up to RS consecutive rows of a strip 64 cells wide (two cells per
 // lane), so that a row's y-neighbours and its lower face coefficient come from the registers
 // of the row before.  A block has 16 warps for up to four rows each, 12 (of 168 registers a
-// thread) for up to eight, and 16 again only where 12 are too few: beside 220 KB of shared
-// memory the L1 cache is too small for spills, and CG at 850^2 takes 7.6 us an iteration
-// with 12 warps and 12.0 with 16.  At the domain's faces a neighbour is the
+// thread) for up to eight, and 16 again (with up to seven where that will do) only where 12
+// are too few: beside 220 KB of shared memory the L1 cache is too small for spills, and CG at
+// 850^2 takes 7.6 us an iteration with 12 warps and 12.0 with 16.  At the domain's faces a neighbour is the
 // cell itself, as the reference's reflecting halo update gives it; only the faces shared by
 // two tiles have halo cells.
 //
@@ -66,8 +66,8 @@ struct ResForm {
     bool cluster;
 };
 constexpr ResForm RES_FORMS[] = {{1, 16, true},  {1, 16, false}, {2, 16, false},
-                                 {4, 16, false}, {8, 12, false}, {8, 16, false}};
-constexpr int RES_FORM_COUNT = 6;
+                                 {4, 16, false}, {8, 12, false}, {7, 16, false}, {8, 16, false}};
+constexpr int RES_FORM_COUNT = 7;
 constexpr int RES_CLUSTER = 16;  // most blocks of a cluster
 constexpr int RES_TRIES = 1 << 18;  // tries at an mbarrier before a wait gives up
 constexpr int RES_POLLS = 1 << 21;  // rounds of polls before a wait gives up (a second or two)
@@ -735,6 +735,80 @@ struct ResTile : GridSum<CL> {
                 ky0 = ky1;
             }
     }
+    // The operand around the warp's rows: the rows below the first and above the last, and in lane k
+    // (8 + k) the cell left (right) of row k.
+    struct Around {
+        Two<T> below, above;
+        T side;
+    };
+    __device__ __forceinline__ Around around() const
+    {
+        Around e;
+        e.below.x = e.below.y = e.above.x = e.above.y = e.side = (T)0;
+        if (rows == 0) return e;
+        const int first = o - 2 * lane, cols = min(64, tw - (x - 2 * lane)), k = lane & 7;
+        const int at = (fl & RF_A0) ? o : first;
+        e.below = ld_two(V + at - ((fl & RF_WFIRST) ? 0 : sx));
+        e.above = ld_two(V + at + (rows - 1) * sx + ((fl & RF_WLAST) ? 0 : sx));
+        if (lane < 16 && k < rows) e.side = V[first + k * sx + (lane < 8 ? -1 : cols)];
+        return e;
+    }
+    // 2D: a sweep whose new operand takes the place of the old one row by row (after every warp has
+    // formed its Around, and before the neighbours' values are collected).  Registers need not hold
+    // the new rows until all warps have read the old ones.  f(k, c, nb0, nb1, kx0, kx1, kx2, ky0, ky1,
+    // out) leaves the row's new cells in out, and they are published.  Every lane of a warp takes
+    // part; those without cells work on lane 0's and store nothing.
+    // Seven rows and 16 warps have no room for the new rows beside two more vectors: with u (PPCG) or
+    // the right-hand side (Chebyshev) in L2 instead, an inner step moved 115 KB per SM through it.
+    // PPCG at 1024^2 91.6 ms a timestep against 107.5, Chebyshev at 1000^2 42.6 against 47.2; the
+    // 12-warp form, which has shared memory for the third vector, gains nothing (800^2: 49.9
+    // against 48.7).
+    template <class F>
+    __device__ __forceinline__ void sweep_over(const Around& e, F&& f) const
+    {
+        if (rows == 0) return;
+        const bool a0 = fl & RF_A0;
+        const int back = a0 ? 0 : 2 * lane;
+        const bool right = 2 * lane + 2 >= min(64, tw - (x - 2 * lane));
+        Two<T> ym = e.below, c = ld_two(V + o - back), ky0 = ld_two(V + oky - back);
+#pragma unroll
+        for (int k = 0; k < RS; ++k)
+            if (k < rows) {
+                const T* vk = cell(k) - back;
+                Two<T> yp = e.above;
+                if (k < rows - 1) yp = ld_two(vk + sx);
+                T l = vk[-1], r = vk[2];
+                const T sl = __shfl_sync(0xffffffffu, e.side, k), sr = __shfl_sync(0xffffffffu, e.side, 8 + k);
+                if (lane == 0) l = sl;
+                if (right) r = sr;
+                const T* kxp = V + okx - back + k * A.p.kxs;
+                const Two<T> kx = ld_two(kxp);
+                const T kx2 = kxp[2];
+                const Two<T> ky1 = ld_two(V + oky - back + (k + 1) * A.p.tws);
+                NbT<T> nb0, nb1;
+                nb0.c = c.x;
+                nb0.xm = (fl & RF_XM) ? c.x : l;
+                nb0.xp = (fl & RF_XP0) ? c.x : c.y;
+                nb0.ym = ym.x;
+                nb0.yp = yp.x;
+                nb1.c = c.y;
+                nb1.xm = c.x;
+                nb1.xp = (fl & RF_XP1) ? c.y : r;
+                nb1.ym = ym.y;
+                nb1.yp = yp.y;
+                nb0.zm = nb0.zp = nb1.zm = nb1.zp = (T)0;
+                Two<T> out;
+                f(k, c, nb0, nb1, kx.x, kx.y, kx2, ky0, ky1, out);
+                __syncwarp();  // every lane has read the row
+                if (a0) {
+                    store(k, out.x, out.y);
+                    publish(k, out.x, out.y);
+                }
+                ym = c;
+                c = yp;
+                ky0 = ky1;
+            }
+    }
     // Adds cell q of row k to a thread's sum; the second cell of a row may not exist.
     __device__ __forceinline__ void add(DD& acc, int k, int q, double v) const
     {
@@ -1151,6 +1225,9 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
     t.load_operand(P::u(a));
     T p[RS][2], un[RS][2];
     const ResOwn<T, RS, CL> b(t, P::rhs(a));
+    // Where the rows of the right-hand side do not stay in registers beside p and the new u, the
+    // sweep works in place, and un holds them for the whole loop.
+    constexpr bool OVER = DIM == 2 && !ResOwn<T, RS, CL>::kept && W > 12;
 #pragma unroll
     for (int k = 0; k < RS; ++k) {
         p[k][0] = p[k][1] = un[k][0] = un[k][1] = (T)0;
@@ -1158,6 +1235,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
     }
     __syncthreads();
     dg.load(t);
+    if constexpr (OVER) b.load(t, un);
     for (;;) {
         const int step = P::fp32 ? s.n_inner - 1 : s.cheby_calc_steps - 1;
         const T al = (T)a.ch_alphas[step], be = (T)a.ch_betas[step];
@@ -1166,23 +1244,37 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
         t.next_exchange();
         Two<T> m;
         m.x = m.y = (T)1;
-        b.load(t, un);
-        t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
-            if (q == 0 && pre) m = t.mi_of(k);
+        auto cell = [&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
             const T wv = dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
             const T rv = un[k][q] - wv;
             const T pv = al * p[k][q] + be * (pre ? (q == 0 ? m.x : m.y) * rv : rv);
             p[k][q] = pv;
-            un[k][q] = nb.c + pv;
-            if (check) t.add(acc, k, q, (double)rv * (double)rv);
-        });
+            if (check && (!OVER || t.on(k))) t.add(acc, k, q, (double)rv * (double)rv);
+            return nb.c + pv;
+        };
+        if constexpr (OVER) {
+            const auto e = t.around();
+            __syncthreads();  // every warp has read the old operand around its rows, and the state
+            t.sweep_over(e, [&](int k, const Two<T>&, const NbT<T>& nb0, const NbT<T>& nb1, T kx0, T kx1, T kx2,
+                                const Two<T>& ky0, const Two<T>& ky1, Two<T>& out) {
+                if (pre && t.on(k)) m = t.mi_of(k);
+                out.x = cell(k, 0, nb0, kx0, kx1, ky0.x, ky1.x, (T)0, (T)0);
+                out.y = cell(k, 1, nb1, kx1, kx2, ky0.y, ky1.y, (T)0, (T)0);
+            });
+        } else {
+            b.load(t, un);
+            t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
+                if (q == 0 && pre) m = t.mi_of(k);
+                un[k][q] = cell(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
+            });
 #pragma unroll
-        for (int k = 0; k < RS; ++k)
-            if (t.on(k)) t.publish(k, un[k][0], un[k][1]);
-        __syncthreads();  // every warp has read the old operand and the state
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) t.publish(k, un[k][0], un[k][1]);
+            __syncthreads();  // every warp has read the old operand and the state
 #pragma unroll
-        for (int k = 0; k < RS; ++k)
-            if (t.on(k)) t.store(k, un[k][0], un[k][1]);
+            for (int k = 0; k < RS; ++k)
+                if (t.on(k)) t.store(k, un[k][0], un[k][1]);
+        }
         auto halo = [&](int first) { t.collect(first, [&](int h, T v) { t.V[t.table()[h].x] = v; }); };
         auto finish = [&](double v) {
             if constexpr (P::fp32) {
@@ -1208,7 +1300,8 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
 #pragma unroll
     for (int k = 0; k < RS; ++k)
         if (t.on(k)) {
-            st_cells(P::u(a), t.gidx(k), t.both(), un[k][0], un[k][1]);
+            const Two<T> c = ld_two(t.cell(k));
+            st_cells(P::u(a), t.gidx(k), t.both(), c.x, c.y);
             st_cells(P::p(a), t.gidx(k), t.both(), p[k][0], p[k][1]);
         }
     RES_EPILOGUE();
@@ -1223,6 +1316,9 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
     t.load_coefs(P::kx(a), P::ky(a), P::kz(a), nullptr);
     t.load_operand(P::p(a));
     constexpr bool PREG = RS * sizeof(T) <= 16;  // p waits in registers, else in its array, for the next outer iteration
+    // Where u does not stay in registers beside r and w, the inner steps work in place, and w holds u
+    // for all of them.
+    constexpr bool OVER = DIM == 2 && !ResOwn<T, RS, CL>::kept && W > 12;
     T r[RS][2], w[RS][2], p[PREG ? RS : 1][2];
     ResOwn<T, RS, CL> u(t, P::u(a));
 #pragma unroll
@@ -1305,7 +1401,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
                 w[k][0] = w[k][0] + alpha * c.x;
                 w[k][1] = w[k][1] + alpha * c.y;
             }
-        u.store(t, w);
+        if constexpr (!OVER) u.store(t, w);
 #pragma unroll
         for (int k = 0; k < RS; ++k)
             if (t.on(k)) set_operand(k, r[k][0] / theta, r[k][1] / theta);
@@ -1314,8 +1410,30 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
         for (int m = 1; m <= inner; ++m) {
             const T al = (T)a.ch_alphas[m - 1], be = (T)a.ch_betas[m - 1];
             const bool last = m == inner;
-            // u += sd first: its rows pass through w, which then takes the new sd.
-            u.load(t, w);
+            if constexpr (OVER) {
+                if (!last) {
+                    const auto e = t.around();
+                    __syncthreads();  // every warp has read the old sd around its rows
+                    t.next_exchange();
+                    t.sweep_over(e, [&](int k, const Two<T>& c, const NbT<T>& nb0, const NbT<T>& nb1, T kx0, T kx1, T kx2,
+                                        const Two<T>& ky0, const Two<T>& ky1, Two<T>& out) {
+                        w[k][0] = w[k][0] + c.x;
+                        w[k][1] = w[k][1] + c.y;
+                        r[k][0] = r[k][0] - dg.smvp(k, 0, nb0, kx0, kx1, ky0.x, ky1.x, (T)0, (T)0);
+                        r[k][1] = r[k][1] - dg.smvp(k, 1, nb1, kx1, kx2, ky0.y, ky1.y, (T)0, (T)0);
+                        out.x = al * c.x + be * r[k][0];
+                        out.y = al * c.y + be * r[k][1];
+                    });
+                    if (exchange() != RN_GO) {
+                        lost = true;
+                        break;
+                    }
+                    continue;
+                }
+            } else {
+                // u += sd first: its rows pass through w, which then takes the new sd.
+                u.load(t, w);
+            }
 #pragma unroll
             for (int k = 0; k < RS; ++k)
                 if (t.on(k)) {
@@ -1327,7 +1445,7 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_ppcg(const __grid_constant__ 
             t.sweep([&](int k, int q, const NbT<T>& nb, T kx0, T kx1, T ky0, T ky1, T kz0, T kz1) {
                 const T rv = r[k][q] - dg.smvp(k, q, nb, kx0, kx1, ky0, ky1, kz0, kz1);
                 r[k][q] = rv;
-                w[k][q] = al * nb.c + be * rv;
+                if constexpr (!OVER) w[k][q] = al * nb.c + be * rv;
                 if (last) t.add(acc, k, q, (double)rv * (double)rv);
             });
             if (last) break;

@@ -77,6 +77,13 @@ def test_cluster_loops_equal_per_call(dim, shape, solver, precond):
     _same(_run(deck, dim, fused=True), _run(deck, dim))
 
 
+@pytest.mark.parametrize("solver", ["chebyshev", "ppcg"])
+@pytest.mark.parametrize("shape", [(1021, 1019), (900, 1100), (1039, 1024)])  # 7 and 8 rows a warp, wide and narrow tiles
+def test_in_place_loops_equal_per_call(shape, solver):
+    deck = _deck(2, shape, solver, False)
+    _same(_run(deck, 2, fused=True), _run(deck, 2))
+
+
 @pytest.mark.parametrize("precond", [False, True])
 @pytest.mark.parametrize("dim,shape", [(d, s) for d in (2, 3) for s in STREAM_SHAPES[d]])
 def test_streaming_cg_equals_per_call(dim, shape, precond):

@@ -45,6 +45,12 @@ __host__ __device__ inline long fidx(const Geom& g, int kk, int jj, int ii)
     return (long)kk + (long)jj * g.pitch + (long)ii * g.page;
 }
 
+// A launch with programmatic stream serialization may start before the launch in front of it has
+// ended: once all its blocks have called let_next_start().  wait_for_previous() waits for its end;
+// nothing it leaves is read, and nothing it uses is written, before that.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ------------------------------------------------------------------ double-double sums
 
 struct DD {

@@ -98,6 +98,7 @@ __device__ __forceinline__ SetupCell setup_cell(const SetupArgs& a, int kk, int 
 // ext_solver_copy_u_ and ext_calculate_2norm_ leave them.
 __global__ void __launch_bounds__(BLOCK) k_setup(const __grid_constant__ SetupArgs a)
 {
+    let_next_start();
     const Geom& g = a.g;
     const Fields& f = a.f;
     DDVec<2> acc;
@@ -168,6 +169,7 @@ __global__ void __launch_bounds__(BLOCK) k_setup(const __grid_constant__ SetupAr
 __global__ void __launch_bounds__(BLOCK) k_settle(FusedArgs a, Fields f, Box inner, SolveState s0, const SolveState* st,
                                                   int p_halo, int energy)
 {
+    wait_for_previous();
     const SolveState& s = st ? *st : s0;
     const Geom& g = a.g;
     const double* pc = a.p[s.par_p];

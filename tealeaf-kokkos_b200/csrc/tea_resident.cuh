@@ -1079,15 +1079,17 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
     extern __shared__ __align__(16) unsigned char s_res_raw[];                                     \
     __shared__ ResShared<CL> sh;                                                                   \
     const FusedArgs& a = A.f;                                                                      \
+    ResTile<T, RS, CL> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                  \
+    wait_for_previous(); /* up to here beside the launch before */                                 \
     if (threadIdx.x == 0) {                                                                        \
         sh.s = A.start ? *A.start : A.s0;                                                          \
+        t.start(RES_SCALE);                                                                        \
     }                                                                                              \
-    ResTile<T, RS, CL> t(A, sh, reinterpret_cast<T*>(s_res_raw));                                  \
-    if (threadIdx.x == 0) t.start(RES_SCALE);                                                      \
-    ResDiag<T, RS, CL> dg;                                                                             \
+    ResDiag<T, RS, CL> dg;                                                                         \
     SolveState& s = sh.s
 
 #define RES_EPILOGUE()                                                                             \
+    let_next_start();                                                                              \
     if constexpr (CL) res_cluster_sync(); /* nothing is on its way to a block that has ended */    \
     else __syncthreads();                                                                          \
     if (blockIdx.x == 0) {                                                                         \

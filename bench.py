@@ -60,16 +60,17 @@ EPS_REL = 1e-10
 SOLVER = "chebyshev"
 METRIC = "s/timestep at rel residual 1e-10 (plain FP64, 2D 4096^2, Chebyshev)"
 WORDS = {  # algorithmic FP64 words per interior cell of one launch
+    "cg_loop": 10.5,   # one iteration: read p, r, Kx, Ky; write p, w; read r, w; write r; every second: p, u; write u
     "cg_sweep_a": 8,   # read p, r, u, Kx, Ky; write u, p, w
     "cg_sweep_b": 3,   # read r, w; write r
     "cheby_iterate": 7,  # read u, u0, p, Kx, Ky; write u', p
     "cheby_pair": 7,  # the same words for two iterations (one pass)
     "cheby_quad": 7,  # four iterations per pass: read u, u0, p, Kx, Ky; write u, p
 }
-KERNEL_IDS = {"cg_sweep_a": 2, "cheby_quad": 11, "cheby_pair": 6, "cg_sweep_b": 5}
+KERNEL_IDS = {"cg_loop": 14, "cheby_quad": 11, "cheby_pair": 6}
 ALL_KERNEL_IDS = {"ppcg_inner": 1, "cg_sweep_a": 2, "cheby_iterate": 3, "jacobi": 4, "cg_sweep_b": 5,
                   "cheby_pair": 6, "cg32_sweep_a": 7, "cg32_sweep_b": 8, "cheby32_pair": 9, "ppcg_pair": 10,
-                  "cheby_quad": 11, "cheby32_quad": 12, "ppcg32_pair": 13}
+                  "cheby_quad": 11, "cheby32_quad": 12, "ppcg32_pair": 13, "cg_loop": 14}
 PROFILES = ROOT / "profiles"
 # The reference's own per-timestep iteration counts on this deck (its Kokkos-OpenMP kernels,
 # oracle/_ref, 30 timesteps at 4096^2), recorded by tests/golden/make_golden_large.py.  They
@@ -328,7 +329,7 @@ def gpu_arm(args, world, precision=0, kernels=True, ws_net=0):
     if kernels:
         # Chebyshev iterations run four per pass, with a two-iteration pass ending at each
         # convergence check (4 + 4 + 2 per 10 iterations once the checks start).
-        share = {"cg_sweep_a": mean_cg * kernel_ms["cg_sweep_a"], "cg_sweep_b": mean_cg * kernel_ms["cg_sweep_b"],
+        share = {"cg_loop": mean_cg * kernel_ms["cg_loop"],
                  "cheby_quad": mean_ch / 5.0 * kernel_ms["cheby_quad"],
                  "cheby_pair": mean_ch / 10.0 * kernel_ms["cheby_pair"]}
         dominant = max(share, key=share.get)
@@ -336,7 +337,7 @@ def gpu_arm(args, world, precision=0, kernels=True, ws_net=0):
     else:
         dominant, alg_bytes = None, None
     # Chebyshev passes: 7 words per pass of four or two iterations (3 passes per 10 iterations).
-    step_words = (WORDS["cg_sweep_a"] + WORDS["cg_sweep_b"]) * mean_cg + WORDS["cheby_pair"] * mean_ch * 0.3
+    step_words = WORDS["cg_loop"] * mean_cg + WORDS["cheby_pair"] * mean_ch * 0.3
     # The same timestep counted in canonical words per iteration (each iteration's arrays
     # once, fusion and temporal blocking not credited): CG 12, Chebyshev 7 (2D).
     canon_words = CANONICAL_WORDS[2]["cg"] * mean_cg + CANONICAL_WORDS[2]["cheby"] * mean_ch
@@ -751,7 +752,7 @@ def learned_arm(args, world):
 # Algorithmic FP64-equivalent words per cell of each fused kernel in 3D (FP32 words count
 # half): the 7-point sweeps read one more coefficient array than their 2D forms.
 WORDS_3D = {"ppcg_inner": 9, "cg_sweep_a": 9, "cheby_iterate": 8, "jacobi": 6, "cg_sweep_b": 3, "cheby_pair": 8,
-            "cg32_sweep_a": 4.5, "cg32_sweep_b": 1.5, "cheby32_pair": 4, "ppcg_pair": 9, "ppcg32_pair": 4.5}
+            "cg32_sweep_a": 4.5, "cg32_sweep_b": 1.5, "cheby32_pair": 4, "ppcg_pair": 9, "ppcg32_pair": 4.5, "cg_loop": 11.5}
 
 
 def ws_predict_3d(args):
@@ -818,7 +819,7 @@ def kernel_only(args):
     # FP32 kernels: their FP32 words counted as half FP64 words.
     words = {"ppcg_inner": 8, "cg_sweep_a": 8, "cheby_iterate": 7, "jacobi": 5, "cg_sweep_b": 3,
              "cheby_pair": 7, "cg32_sweep_a": 4, "cg32_sweep_b": 1.5, "cheby32_pair": 3.5,
-             "ppcg_pair": 8, "cheby_quad": 7, "cheby32_quad": 3.5, "ppcg32_pair": 4}[args.kernel]
+             "ppcg_pair": 8, "cheby_quad": 7, "cheby32_quad": 3.5, "ppcg32_pair": 4, "cg_loop": 10.5}[args.kernel]
     gbs = words * 8 * CELLS * CELLS / (ms.value / 1e3) / 1e9 if ms.value > 0 else None
     print(json.dumps({"kernel": args.kernel, "ms_per_launch": ms.value, "algorithmic_gbs": gbs}))
     lib.ext_finalise_()
@@ -927,12 +928,10 @@ def main():
                      "kernel_frac": {k: WORDS[k] * 8 * CELLS * CELLS / (ms / 1e3) / 1e9 / peak
                                      for k, ms in g["kernel_ms"].items() if ms > 0}},
         "clocks": g["clocks"],
-        # 8 fused launches per four CG iterations (the graph's loop body holds four; the
-        # launches after the last iteration return at once), about 3 per 10 Chebyshev
-        # iterations (passes of four, and of two ending at each convergence check), and
-        # about 27 per-call launches per timestep (set-up, halo updates, the switch, finalise).
-        "gpu_launches": int(sum(8 * ((c + 3) // 4) + (3 * h + 9) // 10 + 27
-                                for c, h in zip(g["cg_steps"], g["cheby_steps"]))),
+        # One launch for the CG loop, about 3 per 10 Chebyshev iterations (passes of four, and
+        # of two ending at each convergence check), and 12 others per timestep (set-up, end,
+        # the switch with the first Chebyshev step).
+        "gpu_launches": int(sum(1 + (3 * h + 9) // 10 + 12 for h in g["cheby_steps"])),
         "cpu_baseline": cpu,
     }
     if e2e:

@@ -71,7 +71,9 @@ int tea_chunk_stream_(const int* chunk, void** stream);
  * iteration, 4 Jacobi sweep, 5 CG sweep B, 6 two Chebyshev iterations in one pass (2D;
  * in 3D one iteration), and the FP32 inner-solve kernels of the precision form: 7 CG
  * sweep A, 8 CG sweep B, 9 two Chebyshev iterations (3D: one); 10 two PPCG inner steps
- * in one pass.  Writes the mean milliseconds per launch. */
+ * in one pass (13: FP32); 11 / 12 four Chebyshev iterations in one pass (2D, FP64 / FP32);
+ * 14 one iteration of the CG loop in the form that the grid's size takes.  Writes the mean
+ * milliseconds per launch (14: per iteration). */
 void tea_kernel_timing_(const int* chunk, const int* kernel, const int* reps, double* ms_per_launch);
 
 /* Host<->device bytes the library has moved for the chunk so far: state tables,
@@ -186,7 +188,7 @@ typedef struct {
 /* Whole implicit solve of one timestep on the device: the control flow of
  * tea_leaf() (tealeaf_2d/tea_solve.f90:36-605, tealeaf_3d/tea_solve.f90:36-653),
  * from the depth-2 halo update of energy/density to ext_solver_finalise_ and the
- * final energy halo update, with the iteration loop captured in CUDA graphs and
+ * final energy halo update, with each iteration loop one kernel or one CUDA graph and
  * the scalar recurrences and convergence test evaluated on the device.  Single
  * chunk only (every face external).  Replaces the per-iteration sequence of
  * ext_cg_calc_w_/ext_cg_calc_ur_/ext_cg_calc_p_/... calls that the Fortran driver

@@ -1,12 +1,15 @@
 // ext_tea_leaf_solve_: the whole implicit solve of one timestep on the device.
 //
-// Follows tea_leaf() (tealeaf_2d/tea_solve.f90:36-605; 3D :36-653) step for step.  The
-// once-per-solve parts -- set-up, the Chebyshev/PPCG switch with its eigenvalue estimate
+// Follows tea_leaf() (tealeaf_2d/tea_solve.f90:36-605; 3D :36-653) step for step.  The set-up of
+// the CG-like solvers and the end are one launch each (tea_ends.cuh); the other once-per-solve
+// parts -- Jacobi's set-up, the Chebyshev/PPCG switch with its eigenvalue estimate
 // (host FP64, tea_eigen.h), the first Chebyshev step and the first PPCG outer iteration,
-// the exact-residual check and the finalise -- call the same per-call kernels as the ext_*
-// entry points.  The iteration loops run as CUDA graphs whose body is one iteration of
-// fused kernels (tea_fused.cuh) inside a while-node; the scalars and the EXIT test live on
-// the device.  Results (fields, iteration counts, errors) equal the per-call sequence that
+// and the exact-residual check -- call the same per-call kernels as the ext_*
+// entry points.  The iteration loops of grids that fit the SMs run as one launch each
+// (tea_resident.cuh), as does the CG loop of larger ones (tea_stream.cuh); the other loops, and
+// all of them where a cooperative launch is not to be had, are CUDA graphs whose body is one
+// iteration of fused kernels (tea_fused.cuh) inside a while-node.  The scalars and the EXIT test
+// live on the device.  Results (fields, iteration counts, errors) equal the per-call sequence that
 // the driver would make bit for bit.
 #include <cuda_runtime.h>
 
@@ -1605,7 +1608,7 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
 // stream between two CUDA events, on the chunk's current fields (their values change).
 // kernel: 1 PPCG inner step, 2 CG/PPCG sweep A, 3 Chebyshev iteration, 4 Jacobi sweep,
 // 10 two PPCG inner steps in one pass, 11/12 four Chebyshev iterations in one pass (2D,
-// FP64/FP32).
+// FP64/FP32), 14 one iteration of the CG loop.
 TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const int* reps, double* ms_per_launch)
 {
     *ms_per_launch = 0.0;
@@ -1614,7 +1617,7 @@ TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const in
     // Coefficient arrays for at least kTimingIters iterations, so that a pass of four
     // Chebyshev iterations reads stored coefficients even before any solve has run.
     constexpr int kTimingIters = 8;
-    Fused* F = ensure_fused(c, kTimingIters);
+    Fused* F = ensure_fused(c, std::max(kTimingIters, *reps));
     if (*kernel >= 7 && !ensure_fp32(c, F)) return;
     FusedArgs a = F->base;
     a.step = 1;
@@ -1718,10 +1721,27 @@ TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const in
         default: stencil<OpJacobi>(F, a, c->stream); break;
         }
     };
-    launch();  // warm-up
-    TEA_CK(cudaEventRecord(e0, c->stream));
-    for (int k = 0; k < *reps; ++k) launch();
-    TEA_CK(cudaEventRecord(e1, c->stream));
+    if (*kernel == 14) {
+        // One launch of the CG loop in the form that the grid's size takes, `reps` iterations of it.
+        for (int k = 0; k < 2; ++k) {
+            SolveState t = saved;
+            t.solver = SOLVER_CG;
+            t.precond = t.pending_p = t.pending_u = t.par_p = t.par_u = 0;
+            t.eps = 0.0;
+            t.n = t.cont = 1;
+            t.max_iters = *reps;
+            *F->h_st = t;
+            TEA_CK(cudaEventRecord(e0, c->stream));
+            const bool ran = launch_loop(c, F, LOOP_CG, 0, false);
+            TEA_CK(cudaEventRecord(e1, c->stream));
+            if (ran) await_loop(c, F);
+        }
+    } else {
+        launch();  // warm-up
+        TEA_CK(cudaEventRecord(e0, c->stream));
+        for (int k = 0; k < *reps; ++k) launch();
+        TEA_CK(cudaEventRecord(e1, c->stream));
+    }
     TEA_CK(cudaEventSynchronize(e1));
     float ms = 0.0f;
     TEA_CK(cudaEventElapsedTime(&ms, e0, e1));

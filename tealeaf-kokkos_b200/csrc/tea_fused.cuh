@@ -15,7 +15,8 @@
 // Scalar recurrences (alpha = rro/pw, beta = rrn/rro, ...) and the loop test of
 // tea_leaf() run in the last block of the reducing kernel, so one iteration is two
 // (CG), one (Chebyshev, Jacobi) or 2 + inner-steps (PPCG) launches, captured in a
-// CUDA graph whose while-node reads the continue flag set there.
+// CUDA graph whose while-node reads the continue flag set there.  Which loops run in one
+// launch instead, and so without these kernels: tea_resident.cuh, tea_stream.cuh.
 #pragma once
 
 #include <type_traits>

@@ -522,6 +522,12 @@ void setup_stream(RingLaunch& L, const Geom& g, int sms, size_t smem)
     const long per_y = std::max<long>(1, warps / per_x);
     L.rows = (int)std::max<long>(8, (g.ny + per_y - 1) / per_y);
 #else
+    // On the largest 3D grids an FP32 iteration is so long that what the streamed loop saves (some
+    // 15 us) is less than what its 12 warps lose in sweep B against the 48 of k_cg32_sweep_b.  us per
+    // iteration, launches of their own and streamed: 256^3 154 and 148, 320^3 344 and 325, 384^3 450
+    // and 467, 448^3 876 and 878, 512^3 1059 and 1130 (400^3, 16 columns past three strips, 798
+    // and 713: given up).
+    if (P::fp32 && (long)g.nx * g.ny * g.nz > ST_FP32_CELLS) return;
     L.rows = ring3_launch(g, sms, ST_GROUPS, strip, ST_TY, sms * ST_GROUPS).rows;
 #endif
     L.blocks = sms;

@@ -19,8 +19,8 @@
 //
 // Measured per CG iteration, launches of their own -> this kernel (HBM time of 10.5 / 11.5 words
 // at the copy peak): 1400^2 41 -> 25.7 us, 2047x2049 78.7 -> 59.3 (53.8), 4096^2 264.5 -> 226 (215),
-// 256^3 294 -> 274 (236), 512^3 2290 -> 2221 (1887); FP32: 2047x2049 47.9 -> 30.5, 4096^2 138 -> 119,
-// 256^3 155 -> 149, 400^3 795 -> 722.  12 warps of 3 rows in flight beat 10 x 4, 14 x 2 and 16 x 2
+// 256^3 294 -> 274 (236), 512^3 2260 -> 2210 (1887); FP32: 2047x2049 47.9 -> 30.5, 4096^2 138 -> 119,
+// 256^3 154 -> 148, 320^3 344 -> 325; larger 3D FP32 grids keep the launches.  12 warps of 3 rows in flight beat 10 x 4, 14 x 2 and 16 x 2
 // (2D, 227 us against 245, 229 and 239 at 4096^2); three groups of 4-row tiles two planes ahead
 // beat 4 x 4 rows x 1 plane, 2 x 6 x 2, 2 x 8 x 1 and 1 x 12 x 2 (3D, 279 us against 339, 291, 321
 // and 289 at 256^3).  Deeper rings where u is not updated and eight rows of sweep B in flight
@@ -48,6 +48,7 @@ constexpr int ST_TY = 4;      // rows of a tile: a group of 4 warps marches thro
 constexpr int ST_GROUPS = 3;  // independent groups of a block
 constexpr int ST_WARPS = ST_TY * ST_GROUPS;
 constexpr int ST_RP = 2;      // planes in flight beyond plane z + 1
+constexpr long ST_FP32_CELLS = 40000000;  // most cells of the FP32 loop
 #endif
 
 constexpr int ST_BACK = 4;  // rows (planes) of sweep B that a thread has in flight

@@ -1475,7 +1475,9 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
         for (int guard = 0; guard < 4 * P->max_iters + 8; ++guard) {
             if (status_store().status == TEA_ERR_CUDA) break;
             const int n = s.n;
-            if ((cheby || ppcg) && switch_check_host(s, n)) {
+            if (running) {
+                running = false;  // the CG loop that followed the set-up: s is its end, not the solve's start
+            } else if ((cheby || ppcg) && switch_check_host(s, n)) {
                 if (s.cheby_calc_steps == 0) {
                     // The switch, tealeaf_2d/tea_solve.f90:184-223, on the host.
                     canonicalize(c, F);
@@ -1574,8 +1576,6 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                 push_state(c, F);
                 if (s.exit_reason == EXIT_CONVERGED || s.exit_reason == EXIT_MAXITER) break;
                 continue;
-            } else if (running) {
-                running = false;  // the CG loop that followed the set-up
             } else {
                 run_loop(c, F, LOOP_CG, 0);
             }

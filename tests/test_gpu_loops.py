@@ -104,3 +104,29 @@ def test_one_launch_fp32_loops_equal_single_launches(dim, shape, solver):
         del os.environ["TEA_B200_NO_GRAPH"]
     assert all(r["corrections"] >= 1 for r in on_chip[0])
     _same(on_chip, single)
+
+
+def _spec_deck(dim, shape, states=6, **kw):
+    deck = tea.seeded_deck(tea.DeckSpec(dim=dim, cells=8, states=states, end_step=1, summary_frequency=1, **kw))
+    for axis, n in zip("xyz", shape):
+        deck = deck.replace(f"{axis}_cells=8\n", f"{axis}_cells={n}\n")
+    return deck
+
+
+def _same_step(a, b, what):
+    for k in FIELDS:
+        assert same(a[0][0][k], b[0][0][k]), (what, k, a[0][0][k], b[0][0][k])
+    for f in a[1]:
+        assert np.array_equal(a[1][f], b[1][f], equal_nan=True), (what, f)
+
+
+@pytest.mark.parametrize("solver", ["chebyshev", "ppcg"])
+@pytest.mark.parametrize("dim,shape", [(2, (10, 10)), (2, (131, 33)), (2, (300, 200)), (2, (1101, 1003)), (3, (17, 7, 9))])
+def test_solve_that_ends_in_its_cg_phase_equals_per_call(dim, shape, solver):
+    # Converged from above the switch's error of 1, or out of iterations where it would switch: no switch follows.
+    dt = 4.0 * (10.0 / max(shape)) ** 2
+    for eps, iters in ((0.9, (400,)), (1e-12, range(3, 30))):
+        for max_iters in iters:
+            deck = _spec_deck(dim, shape, seed=5, solver=solver, dt=dt, eps=eps, max_iters=max_iters, presteps=3,
+                              inner_steps=4)
+            _same_step(_run(deck, dim, fused=True), _run(deck, dim), (eps, max_iters))

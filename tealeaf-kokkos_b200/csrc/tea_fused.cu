@@ -10,7 +10,7 @@
 // all of them where a cooperative launch is not to be had, are CUDA graphs whose body is one
 // iteration of fused kernels (tea_fused.cuh) inside a while-node.  The scalars and the EXIT test
 // live on the device.  Results (fields, iteration counts, errors) equal the per-call sequence that
-// the driver would make bit for bit.
+// the driver would make bit for bit, as far as a double-double sum rounds the same in another order.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -544,7 +544,7 @@ void setup_resident(Chunk* c, Fused* F, int sms)
     const size_t smem = optin > 2048 ? (size_t)optin - 2048 : 0;  // less the kernels' static part
     sms = std::min(sms, 255);  // the arrivals at a sum are counted in a byte
     if (!coop || c->red.max_blocks < sms) return;
-    const size_t sums = RES_SUM_WORDS * sizeof(unsigned long long);
+    const size_t sums = RES_SUM_BYTES;
     TEA_CK(cudaMalloc(&F->sums, sums));
     if (!F->sums) return;
     TEA_CK(cudaMemsetAsync(F->sums, 0, sums, c->stream));

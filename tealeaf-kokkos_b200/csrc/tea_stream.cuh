@@ -65,7 +65,8 @@ struct StreamRing {
     static constexpr int parts = ST_GROUPS, rows = (ST_RP + 2) * (2 * (ST_TY + 2) + 5 * ST_TY + 1);
 #endif
     static constexpr int elems = rows * RingGeom<T>::WIDTH;
-    static constexpr size_t bytes = (size_t)parts * elems * sizeof(T);
+    static constexpr size_t bytes = (size_t)parts * elems * sizeof(T) + 16;  // of which ring_start() leaves 0 or 16
+    static_assert(RingGeom<T>::WIDTH * sizeof(T) % 32 == 0 && RingGeom<T>::OFF * sizeof(T) == 16, "see ring_start");
 };
 
 // One iteration's operands: p and the new p's buffer (which holds the p before), q = z or r
@@ -468,6 +469,15 @@ struct StreamP<ResF32> {
     __device__ static float* p(const FusedArgs& a, int b) { return a.p32[b]; }
 };
 
+// A row's strip starts 16 bytes behind the row.  It has to start on 32 bytes, as the sectors that the
+// copies bring do (16 bytes off, an iteration takes 6-9 % longer), wherever the kernel's static part ends.
+// (Not by the array's alignment: all kernels of the file share it, and others' rings would move.)
+template <class T>
+__device__ __forceinline__ T* ring_start(unsigned char* raw)
+{
+    return reinterpret_cast<T*>(raw + ((16 - res_shared(raw)) & 31));
+}
+
 template <class P>
 __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_constant__ StreamArgs A)
 {
@@ -484,7 +494,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_con
     constexpr int warps = ST_WARPS / StreamRing<T>::parts;  // that share a ring
     const int part = sum.warp / warps;
     const int first = blockIdx.x * StreamRing<T>::parts + part, stride = gridDim.x * StreamRing<T>::parts;
-    T* ring = reinterpret_cast<T*>(s_stream_raw) + part * StreamRing<T>::elems;
+    T* ring = ring_start<T>(s_stream_raw) + part * StreamRing<T>::elems;
     __syncthreads();
     const bool pre = !P::fp32 && s.precond;
     int par = s.par_p, waiting = 0;  // p's buffer, steps of u not yet taken

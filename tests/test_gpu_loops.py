@@ -130,3 +130,75 @@ def test_solve_that_ends_in_its_cg_phase_equals_per_call(dim, shape, solver):
             deck = _spec_deck(dim, shape, seed=5, solver=solver, dt=dt, eps=eps, max_iters=max_iters, presteps=3,
                               inner_steps=4)
             _same_step(_run(deck, dim, fused=True), _run(deck, dim), (eps, max_iters))
+
+
+# ------------------------------------------------------------- sums that cancel or collapse
+
+def _outcome(deck, dim, **kw):
+    """The run's records and fields, or the error that it ended with."""
+    try:
+        return _run(deck, dim, **kw)
+    except RuntimeError as e:
+        return str(e)
+
+
+def _same_outcome(a, b, what):
+    if isinstance(a, str) or isinstance(b, str):
+        # Only the eigenvalue estimate of a Chebyshev or PPCG solve may fail, and then on both paths.
+        assert isinstance(a, str) and isinstance(b, str) and "status 5" in a and ("status 5" in b or "eigenvalues" in b), \
+            (what, a, b)
+        return
+    _same_step(a, b, what)
+
+
+def _single(deck, dim, **kw):
+    os.environ["TEA_B200_NO_GRAPH"] = "1"
+    try:
+        return _outcome(deck, dim, **kw)
+    finally:
+        del os.environ["TEA_B200_NO_GRAPH"]
+
+
+# One block, a cluster, and many blocks with one, four and seven rows a warp.
+STIFF_SHAPES = [(2, (5, 5)), (2, (10, 10)), (2, (16, 16)), (2, (33, 20)), (2, (23, 2)), (3, (6, 5, 7)), (2, (131, 97)),
+                (2, (300, 200)), (3, (31, 30, 29))]
+
+
+@pytest.mark.parametrize("dt", [1e5, 1e6, 1e7])
+@pytest.mark.parametrize("dim,shape", STIFF_SHAPES)
+def test_sums_with_cancelling_terms_equal_per_call(dim, shape, dt):
+    # Stiff steps: the terms of p.w are far larger than p.w.
+    for seed in range(4):
+        for solver, precond in (("cg", False), ("cg", True), ("ppcg", False)):
+            deck = _spec_deck(dim, shape, seed=seed, solver=solver, dt=dt, eps=1e-6, max_iters=150, presteps=20,
+                              inner_steps=5, preconditioner=precond)
+            _same_outcome(_outcome(deck, dim, fused=True), _outcome(deck, dim), (seed, solver, precond))
+
+
+@pytest.mark.parametrize("dim,shape", [(2, (700, 650)), (2, (1023, 1009)), (2, (1101, 1003)), (3, (101, 99, 97))])
+def test_large_sums_with_cancelling_terms_equal_per_call(dim, shape):
+    for precond in (False, True):
+        deck = _spec_deck(dim, shape, seed=3, solver="cg", dt=1e5, eps=1e-6, max_iters=60, preconditioner=precond)
+        _same_outcome(_outcome(deck, dim, fused=True), _outcome(deck, dim), precond)
+
+
+@pytest.mark.parametrize("dt", [1e3, 1e5])
+@pytest.mark.parametrize("dim,shape", STIFF_SHAPES + [(2, (1101, 1003))])
+def test_fp32_sums_with_cancelling_terms_equal_single_launches(dim, shape, dt):
+    for solver in ("cg", "chebyshev", "ppcg"):
+        deck = _spec_deck(dim, shape, seed=1, solver=solver, dt=dt, eps=1e-6, max_iters=100, presteps=20, inner_steps=6)
+        kw = {"fused": True, "precision": tea.PRECISION_FP32_REFINED}
+        _same_outcome(_outcome(deck, dim, **kw), _single(deck, dim, **kw), solver)
+
+
+@pytest.mark.parametrize("dt", [0.004, 0.35, 30.0])
+@pytest.mark.parametrize("dim,shape", [(2, (2, 2)), (2, (2, 3)), (2, (3, 3)), (2, (6, 2)), (2, (17, 2)), (3, (2, 2, 2)),
+                                       (3, (2, 3, 2))])
+def test_sums_that_collapse_equal_per_call(dim, shape, dt):
+    # CG ends in as many iterations as the operator has eigenvalues, with a fall of r.r by 100 bits in one of
+    # them; Jacobi's first sum is far below the error that the loop starts from.
+    for seed in range(4):
+        for solver, precond in (("cg", False), ("cg", True), ("chebyshev", False), ("jacobi", False)):
+            deck = _spec_deck(dim, shape, states=4, seed=seed, solver=solver, dt=dt, eps=1e-60, max_iters=40, presteps=3,
+                              preconditioner=precond)
+            _same_outcome(_outcome(deck, dim, fused=True), _outcome(deck, dim), (seed, solver, precond))

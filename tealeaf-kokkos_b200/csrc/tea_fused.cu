@@ -609,7 +609,8 @@ const void* res_kernel(int kind, int form)
 
 // Launch loop `kind` as one on-chip kernel from the host's state or, with `started`, from the state
 // that the set-up leaves in d_start (the host's has the same flags); false when the grid, the
-// loop or the state is not of a form it takes (then the loop runs as a graph).
+// loop or the state is not of a form it takes (then the loop runs as a graph).  The loop writes its
+// final state to the host's record: from the launch to await_loop() the host leaves it alone.
 bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started)
 {
     const SolveState& s = *F->h_st;
@@ -627,6 +628,8 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started
     A.elems = (long)c->field_elems;
     A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->m_st)};
     A.epoch = F->epoch;
+    // More epochs than the loop can use: two rim exchanges and one per inner step an iteration.
+    const unsigned long long epochs = (unsigned long long)(s.max_iters + 2) * (inner_steps + 4) + 16;
     const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
     void* args[] = {&A};
     cudaError_t launched;
@@ -645,8 +648,7 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started
         F->res[0].blocks = F->res[1].blocks = F->res32.blocks = 0;
         return false;
     }
-    // More epochs than the loop can use: two rim exchanges and one per inner step an iteration.
-    F->epoch += (unsigned long long)(s.max_iters + 2) * (inner_steps + 4) + 16;
+    F->epoch += epochs;
     F->sum_set ^= 1;
     return true;
 }
@@ -1274,10 +1276,12 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
     bool running = false, settled = false;
     if (cg_like && coefficient >= 1 && c->g.nx > 1 && c->g.ny > 1 && (DIM == 2 || c->g.nz > 1)) {
         launch_setup(c, F, P, s);
+        const SolveState unused = s;  // k_settle takes the loop's state from device memory
         running = !c->ws && P->precision == TEA_PRECISION_FP64 && launch_loop(c, F, LOOP_CG, 0, true);
         if (running && solver == TEA_SOLVER_CG) {
             const EarlyLaunch E(F->point_blocks, dim3(TILE_X, TILE_Y), 0, c->stream, false);
-            TEA_CK(cudaLaunchKernelEx(&E.L, k_settle, F->base, c->f, c->inner, s, (const SolveState*)F->d_st, 1, 1));
+            TEA_CK(cudaLaunchKernelEx(&E.L, k_settle, F->base, c->f, c->inner, unused, (const SolveState*)F->d_st, 1,
+                                      1));
             settled = true;
         }
         if (running) {

@@ -628,8 +628,10 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started
     A.elems = (long)c->field_elems;
     A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->m_st)};
     A.epoch = F->epoch;
-    // More epochs than the loop can use: two rim exchanges and one per inner step an iteration.
-    const unsigned long long epochs = (unsigned long long)(s.max_iters + 2) * (inner_steps + 4) + 16;
+    // More epochs than the loop can use: two rim exchanges an iteration and, in a PPCG loop, one per inner
+    // step (the other solvers' parameters may hold any number there).
+    const unsigned long long steps = kind == LOOP_PPCG || kind == LOOP_PPCG32 ? inner_steps : 0;
+    const unsigned long long epochs = ((unsigned long long)s.max_iters + 2) * (steps + 4) + 16;
     const void* k = fp32 ? res_kernel<ResF32>(kind, p.form) : res_kernel<ResF64>(kind, p.form);
     void* args[] = {&A};
     cudaError_t launched;

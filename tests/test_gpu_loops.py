@@ -202,3 +202,18 @@ def test_sums_that_collapse_equal_per_call(dim, shape, dt):
             deck = _spec_deck(dim, shape, states=4, seed=seed, solver=solver, dt=dt, eps=1e-60, max_iters=40, presteps=3,
                               preconditioner=precond)
             _same_outcome(_outcome(deck, dim, fused=True), _outcome(deck, dim), (seed, solver, precond))
+
+
+@pytest.mark.parametrize("inner_steps", [0, -4, -8])
+@pytest.mark.parametrize("dim,shape", [(2, (300, 200)), (3, (48, 48, 48))])
+def test_chebyshev_solves_do_not_depend_on_inner_steps(dim, shape, inner_steps):
+    # Only a PPCG solve has inner steps: the rim words' epochs grow by the exchanges of the loop that runs.
+    deck = _deck(dim, shape, "chebyshev", False).replace("end_step=2", "end_step=6")
+    own = [ln for ln in deck.splitlines() if ln.startswith("tl_ppcg_inner_steps")][0]
+    a = _run(deck.replace(own, f"tl_ppcg_inner_steps={inner_steps}"), dim, fused=True)
+    b = _run(deck, dim)
+    for x, y in zip(a[0], b[0], strict=True):
+        for k in FIELDS:
+            assert same(x[k], y[k]), (x["step"], k, x[k], y[k])
+    for f in a[1]:
+        assert np.array_equal(a[1][f], b[1][f]), f

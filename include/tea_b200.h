@@ -73,7 +73,7 @@ int tea_chunk_stream_(const int* chunk, void** stream);
  * sweep A, 8 CG sweep B, 9 two Chebyshev iterations (3D: one); 10 two PPCG inner steps
  * in one pass (13: FP32); 11 / 12 four Chebyshev iterations in one pass (2D, FP64 / FP32);
  * 14 one iteration of the CG loop in the form that the grid's size takes.  Writes the mean
- * milliseconds per launch (14: per iteration). */
+ * milliseconds per launch (14: per iteration; 0 where that loop is not one launch). */
 void tea_kernel_timing_(const int* chunk, const int* kernel, const int* reps, double* ms_per_launch);
 
 /* Host<->device bytes the library has moved for the chunk so far: state tables,

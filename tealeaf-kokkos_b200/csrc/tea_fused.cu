@@ -1103,16 +1103,17 @@ bool launch_loop(Chunk* c, Fused* F, int kind, int inner_steps, bool started)
     return launch_resident(c, F, kind, inner_steps, started) || launch_stream(c, F, kind, started);
 }
 
-// Waits for a loop launched by launch_loop, which has left its final state in the host's record.
-void await_loop(Chunk* c, Fused* F)
+// Waits for a loop launched by launch_loop, which has left its final state in the host's record; false
+// when its blocks gave up waiting for one another.
+bool await_loop(Chunk* c, Fused* F)
 {
     sync(c);
     c->d2h_bytes += sizeof(SolveState);
-    if (*(volatile int*)fail_of(F->h_st)) {
-        set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of a loop lost one another");
-        *fail_of(F->h_st) = 0;
-        TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
-    }
+    if (!*(volatile int*)fail_of(F->h_st)) return true;
+    set_status(TEA_ERR_CUDA, "ext_tea_leaf_solve_: the blocks of a loop lost one another");
+    *fail_of(F->h_st) = 0;
+    TEA_CK(cudaMemsetAsync(F->sums, 0, RES_SUM_WORDS * sizeof(unsigned long long), c->stream));
+    return false;
 }
 
 // Run loop `kind` from the current state until its exit; the host state is refreshed.
@@ -1733,9 +1734,11 @@ TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const in
         default: stencil<OpJacobi>(F, a, c->stream); break;
         }
     };
+    bool ran = true;
     if (*kernel == 14) {
-        // One launch of the CG loop in the form that the grid's size takes, `reps` iterations of it.
-        for (int k = 0; k < 2; ++k) {
+        // One launch of the CG loop in the form that the grid's size takes, `reps` iterations of it; 0 ms
+        // where the loop is a graph, or failed.
+        for (int k = 0; k < 2 && ran; ++k) {
             SolveState t = saved;
             t.solver = SOLVER_CG;
             t.precond = t.pending_p = t.pending_u = t.par_p = t.par_u = 0;
@@ -1744,9 +1747,9 @@ TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const in
             t.max_iters = *reps;
             *F->h_st = t;
             TEA_CK(cudaEventRecord(e0, c->stream));
-            const bool ran = launch_loop(c, F, LOOP_CG, 0, false);
+            ran = launch_loop(c, F, LOOP_CG, 0, false);
             TEA_CK(cudaEventRecord(e1, c->stream));
-            if (ran) await_loop(c, F);
+            ran = ran && await_loop(c, F);
         }
     } else {
         launch();  // warm-up
@@ -1757,7 +1760,7 @@ TEA_EXPORT void tea_kernel_timing_(const int* chunk, const int* kernel, const in
     TEA_CK(cudaEventSynchronize(e1));
     float ms = 0.0f;
     TEA_CK(cudaEventElapsedTime(&ms, e0, e1));
-    *ms_per_launch = (double)ms / *reps;
+    if (ran) *ms_per_launch = (double)ms / *reps;
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     *F->h_st = saved;

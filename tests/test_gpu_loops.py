@@ -217,3 +217,33 @@ def test_chebyshev_solves_do_not_depend_on_inner_steps(dim, shape, inner_steps):
             assert same(x[k], y[k]), (x["step"], k, x[k], y[k])
     for f in a[1]:
         assert np.array_equal(a[1][f], b[1][f]), f
+
+
+def _chunk(dim, shape):
+    """A chunk with random density and energy."""
+    lib = tea.cuda_library(dim)
+    chunk = tea.ExtChunk(lib, dim, *shape)
+    chunk.initialise(0.0, 0.0, 10.0 / shape[0], 10.0 / shape[1], 0.0, 10.0 / (shape[2] if dim == 3 else 1))
+    rng = np.random.default_rng(7)
+    chunk.write("density", rng.uniform(0.5, 20.0, (chunk.Z, chunk.Y, chunk.X)))
+    chunk.write("energy1", rng.uniform(1.0, 25.0, (chunk.Z, chunk.Y, chunk.X)))
+    return lib, chunk
+
+
+@pytest.mark.parametrize("dim,shape", [(2, (40, 30)), (2, (1101, 1003)), (3, (20, 20, 20))])
+def test_cg_loop_timing_is_zero_without_a_loop(dim, shape):
+    def timing():
+        lib, chunk = _chunk(dim, shape)
+        try:
+            ms = ctypes.c_double(-1.0)
+            lib.tea_kernel_timing_(chunk.cid, ctypes.byref(ctypes.c_int(14)), ctypes.byref(ctypes.c_int(5)), ctypes.byref(ms))
+            return ms.value
+        finally:
+            lib.ext_finalise_()
+
+    assert timing() > 0.0
+    os.environ["TEA_B200_NO_GRAPH"] = "1"
+    try:
+        assert timing() == 0.0
+    finally:
+        del os.environ["TEA_B200_NO_GRAPH"]

@@ -76,6 +76,12 @@ int tea_chunk_stream_(const int* chunk, void** stream);
  * milliseconds per launch (14: per iteration; 0 where that loop is not one launch). */
 void tea_kernel_timing_(const int* chunk, const int* kernel, const int* reps, double* ms_per_launch);
 
+/* Test hook: how often the blocks of a one-launch loop look for what they wait for in global
+ * memory before the loop gives up and the solve ends in TEA_ERR_CUDA; from the chunk's next
+ * solve on.  Negative: the default, a second or two.  0: a wait that is not over at the first
+ * look has run out. */
+void tea_poll_limit_(const int* chunk, const int* polls);
+
 /* Host<->device bytes the library has moved for the chunk so far: state tables,
  * coefficients, scalars and results (the field arrays never leave the device). */
 int tea_transfer_bytes_(const int* chunk, long long* h2d, long long* d2h);

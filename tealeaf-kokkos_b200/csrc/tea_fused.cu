@@ -92,6 +92,7 @@ struct Fused {
     unsigned long long* sums = nullptr;
     unsigned long long epoch = 0;
     int sum_set = 0;
+    int polls = RES_POLLS;  // the blocks' patience with one another
     RingLaunch stream, stream32;  // k_stream_cg in FP64 and FP32 (blocks 0: not used)
 };
 
@@ -626,7 +627,7 @@ bool launch_resident(Chunk* c, Fused* F, int kind, int inner_steps, bool started
     A.host = F->m_st;
     A.rim = F->rim;
     A.elems = (long)c->field_elems;
-    A.sum = {F->sums, F->sum_set, p.blocks, fail_of(F->m_st)};
+    A.sum = {F->sums, F->sum_set, p.blocks, F->polls, fail_of(F->m_st)};
     A.epoch = F->epoch;
     // More epochs than the loop can use: two rim exchanges an iteration and, in a PPCG loop, one per inner
     // step (the other solvers' parameters may hold any number there).
@@ -668,7 +669,7 @@ bool launch_stream(Chunk* c, Fused* F, int kind, bool started)
     A.start = started ? F->d_start : nullptr;
     A.s0 = s;
     A.host = F->m_st;
-    A.sum = {F->sums, F->sum_set, L.blocks, fail_of(F->m_st)};
+    A.sum = {F->sums, F->sum_set, L.blocks, F->polls, fail_of(F->m_st)};
     A.seg = L.rows;
     const void* k = fp32 ? (const void*)k_stream_cg<ResF32> : (const void*)k_stream_cg<ResF64>;
     const size_t bytes = fp32 ? StreamRing<float>::bytes : StreamRing<double>::bytes;
@@ -1615,6 +1616,13 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
     R->warm_start_used = ws_used;
     R->warm_r0_plain = ws_r0_plain;
     R->warm_r0_guess = ws_r0_guess;
+}
+
+// The blocks' patience with one another in the one-launch loops (but for clusters), for the tests.
+TEA_EXPORT void tea_poll_limit_(const int* chunk, const int* polls)
+{
+    Chunk* c = get_chunk(chunk);
+    if (c) ensure_fused(c, 1)->polls = *polls < 0 ? RES_POLLS : *polls;
 }
 
 // Measurement hook: `reps` back-to-back launches of one fused kernel on the chunk's

@@ -113,6 +113,7 @@ struct SumArgs {
     unsigned long long* sums;  // RES_SUM_WORDS and the slots; this launch's set is zero, the other set's words
     int set;                   // are cleared for the next launch
     int blocks;                // at most 255 (the arrivals are counted in a byte)
+    int polls;                 // rounds of polls before a wait gives up
     int* fail;
 };
 
@@ -155,11 +156,12 @@ __device__ __forceinline__ ResWord res_get(const ResWord* p)
 }
 // The value of a word once it carries `tag`; after the poll limit, or when another block has
 // given up, sets gave_up and returns whatever is there.
-__device__ __forceinline__ unsigned long long res_wait(const ResWord* q, unsigned long long tag, int* fail, bool& gave_up)
+__device__ __forceinline__ unsigned long long res_wait(const ResWord* q, unsigned long long tag, int polls, int* fail,
+                                                       bool& gave_up)
 {
     ResWord w = res_get(q);
     for (int k = 0; w.tag != tag; ++k) {
-        if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)fail != 0)) {
+        if (k >= polls || ((k & 1023) == 1023 && *(volatile int*)fail != 0)) {
             gave_up = true;
             break;
         }
@@ -509,7 +511,7 @@ struct GridSum {
         __syncwarp();
         now += add;
         for (int k = 0; __any_sync(0xffffffffu, has && (int)((now - old) >> 56) != sa.blocks); ++k) {
-            if ((k & 1023) == 1023 && (k >= RES_POLLS || *(volatile int*)sa.fail != 0)) {
+            if (k >= sa.polls || ((k & 1023) == 1023 && *(volatile int*)sa.fail != 0)) {
                 gave_up = true;
                 break;
             }
@@ -995,7 +997,7 @@ struct ResTile : GridSum<CL> {
         }
         const ResWord* q = A.rim + (tag & 1) * A.elems + kLeadPad;
         for (int h = (warp - first) * 32 + lane; h < nh; h += (nw - first) * 32) {
-            put(h, res_value<T>(res_wait(q + table()[h].y, tag, sa.fail, gave_up)));
+            put(h, res_value<T>(res_wait(q + table()[h].y, tag, sa.polls, sa.fail, gave_up)));
         }
     }
 };

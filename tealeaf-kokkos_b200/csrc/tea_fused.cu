@@ -543,6 +543,7 @@ void setup_resident(Chunk* c, Fused* F, int sms)
     TEA_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device));
     TEA_CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device));
     const size_t smem = optin > 2048 ? (size_t)optin - 2048 : 0;  // less the kernels' static part
+    static_assert(sizeof(ResShared<true>) <= 2048, "the static part");
     sms = std::min(sms, 255);  // the arrivals at a sum are counted in a byte
     if (!coop || c->red.max_blocks < sms) return;
     const size_t sums = RES_SUM_BYTES;

@@ -78,7 +78,8 @@ constexpr ResForm RES_FORMS[] = {{1, 16, true},  {1, 16, false}, {2, 16, false},
                                  {4, 16, false}, {8, 12, false}, {7, 16, false}, {8, 16, false}};
 constexpr int RES_FORM_COUNT = 7;
 constexpr int RES_CLUSTER = 16;  // most blocks of a cluster
-constexpr int RES_TRIES = 1 << 18;  // tries at an mbarrier before a wait gives up
+constexpr unsigned long long RES_BAR_NS = 2000000000ull;  // a wait at an mbarrier gives up after this time
+constexpr unsigned long long RES_DRAIN_NS = 1000000ull;   // what is on its way in a cluster is given to arrive
 constexpr int RES_POLLS = 1 << 21;  // rounds of polls before a wait gives up (a second or two)
 constexpr int RES_LIMBS = 4;         // limbs of a sum, and one word of flags
 constexpr int RES_SUM_STRIDE = 32;   // 64-bit words between two sums: a sum's words share a line
@@ -221,13 +222,25 @@ __device__ __forceinline__ bool res_arrived(unsigned bar, unsigned phase)
         : "memory");
     return ok != 0;
 }
-// Waits for a phase of an mbarrier; gives up as res_wait does.
+__device__ __forceinline__ unsigned long long res_now()
+{
+    unsigned long long ns;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(ns));
+    return ns;
+}
+// Waits for a phase of an mbarrier; gives up as res_wait does, but by the clock: the hardware chooses how
+// long a try takes.
 __device__ __forceinline__ void res_wait_bar(unsigned bar, unsigned phase, int* fail, bool& gave_up)
 {
+    unsigned long long from = 0;
     for (int k = 0; !res_arrived(bar, phase); ++k)
-        if ((k & 1023) == 1023 && (k >= RES_TRIES || *(volatile int*)fail != 0)) {
-            gave_up = true;
-            break;
+        if ((k & 63) == 63) {
+            const unsigned long long now = res_now();
+            if (from == 0) from = now;
+            if (now - from >= RES_BAR_NS || *(volatile int*)fail != 0) {
+                gave_up = true;
+                break;
+            }
         }
 }
 __device__ __forceinline__ void res_cluster_sync()
@@ -245,6 +258,7 @@ struct ClusterShared {
     alignas(16) unsigned long long sums[2][RES_CLUSTER][4];
     unsigned long long sum_bar[2], rim_bar[2];
     ResFace face[6];
+    int gone;  // a block of the cluster has given up
 };
 template <>
 struct ClusterShared<false> {
@@ -691,6 +705,7 @@ struct ResTile : GridSum<CL> {
                     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(res_shared(&ss.sum_bar[k])) : "memory");
                     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(res_shared(&ss.rim_bar[k])) : "memory");
                 }
+                ss.gone = 0;
                 asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
             }
             if (threadIdx.x < 6) {
@@ -709,6 +724,25 @@ struct ResTile : GridSum<CL> {
                 }
             }
             res_cluster_sync();
+        }
+    }
+    // The end of a cluster's loop: nothing may be on its way to a block that has ended.  Where no wait has
+    // given up, each block has waited for all that was sent to it.  Else no instruction waits for the
+    // stores still under way: once no block sends any more, they are given a thousand times what they take.
+    __device__ void leave() const
+    {
+        if constexpr (CL) {
+            if (ss.lost && (int)threadIdx.x < sa.blocks)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(res_remote(res_shared(&ss.gone), threadIdx.x)), "r"(1)
+                             : "memory");
+            __syncwarp();
+            res_cluster_sync();
+            if (*(volatile int*)&ss.gone) {
+                const unsigned long long from = res_now();
+                while (res_now() - from < RES_DRAIN_NS) __nanosleep(1000);
+                __syncwarp();
+                res_cluster_sync();
+            }
         }
     }
     // Halo cells at face f of the tile of block (bx, by, bz), w x h x e cells.
@@ -1202,7 +1236,7 @@ __device__ __forceinline__ void cg_note_rr(const FusedArgs& a, SolveState& s, do
 
 #define RES_EPILOGUE()                                                                             \
     let_next_start();                                                                              \
-    if constexpr (CL) res_cluster_sync(); /* nothing is on its way to a block that has ended */    \
+    if constexpr (CL) t.leave();                                                                   \
     else __syncthreads();                                                                          \
     if (blockIdx.x == 0) {                                                                         \
         if (threadIdx.x == 0) *a.st = *A.host = s;                                                 \

@@ -1118,19 +1118,20 @@ bool await_loop(Chunk* c, Fused* F)
     return false;
 }
 
-// Run loop `kind` from the current state until its exit; the host state is refreshed.
-void run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
+// Run loop `kind` from the current state until its exit; the host state is refreshed.  True when it ran
+// as one launch.
+bool run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
 {
     F->h_st->cont = 1;  // the body runs at least once (the while node's default)
     if (launch_loop(c, F, kind, inner_steps, false)) {
         await_loop(c, F);
-        return;
+        return true;
     }
     push_state(c, F);
     if (F->use_graph && build_loop(c, F, kind, inner_steps)) {
         TEA_CK(cudaGraphLaunch(F->loops[kind].exec, c->stream));
         pull_state(c, F);
-        return;
+        return false;
     }
     // Without graphs: one iteration per launch sequence, the exit flag read back each time.
     FusedArgs a = F->base;
@@ -1139,6 +1140,7 @@ void run_loop(Chunk* c, Fused* F, int kind, int inner_steps)
         pull_state(c, F);
         if (!F->h_st->cont || status_store().status == TEA_ERR_CUDA) break;
     }
+    return false;
 }
 
 // Host mirror of end_iteration() for the iterations run by per-call kernels.
@@ -1191,6 +1193,50 @@ void canonicalize(Chunk* c, Fused* F, bool refresh_p = true, bool energy = false
     TEA_CK(cudaGetLastError());
     s.pending_p = s.pending_u = 0;
     s.par_p = s.par_u = 0;
+}
+
+// After a Chebyshev loop that CG takes over from (the error rose above 1): the residual of its last
+// iteration, which the per-call kernels would have left in r and the loops do not store.  An on-chip loop
+// (from `first_step` on) has left u and p as they were, the other forms have the ones before their last
+// pass in the second buffers: the iterations since run again by the per-call kernels, and end in the
+// same u and p.
+void restore_residual(Chunk* c, Fused* F, const int* chunk, bool on_chip, int first_step)
+{
+    SolveState& s = *F->h_st;
+    // Inner u and p from one of their buffers to the canonical ones, with u's halo.
+    auto settle = [&](const FusedArgs& a, int par_u, int par_p) {
+        SolveState t = {};
+        t.par_u = par_u;
+        t.par_p = par_p;
+        k_settle<<<F->point_blocks, dim3(TILE_X, TILE_Y), 0, c->stream>>>(a, c->f, c->inner, t, nullptr, 0, 0);
+        TEA_CK(cudaGetLastError());
+    };
+    FusedArgs a = F->base;
+    if (!on_chip && s.last_pass == 1) {
+        // One iteration, p in place: r = u0 - A u on the u before it.
+        if (!s.par_u) {
+            TEA_CK(cudaMemcpyAsync(F->alt[2], c->alloc[F_U], c->field_elems * sizeof(double), cudaMemcpyDeviceToDevice,
+                                   c->stream));
+            settle(a, 1, s.par_p);
+            a.u[1] = a.sd[1];
+        } else {
+            settle(a, 0, s.par_p);
+        }
+        ext_calculate_residual_(chunk);
+        settle(a, 1, 0);
+    } else {
+        if (on_chip) {
+            settle(a, 0, 0);
+        } else {
+            settle(a, s.par_u ^ 1, s.par_p ^ 1);
+            first_step = s.cheby_calc_steps - s.last_pass;
+        }
+        for (int step = first_step; step < s.cheby_calc_steps; ++step) {
+            ext_cheby_solver_iterate_(chunk, &step);
+            halo(c, {4}, 1);
+        }
+    }
+    s.par_u = s.par_p = 0;
 }
 
 // The set-up of a CG, Chebyshev or PPCG solve in one launch; `s` is the starting state but for
@@ -1566,7 +1612,9 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                     if (s.exit_reason == EXIT_CONVERGED || s.exit_reason == EXIT_MAXITER) break;
                     continue;
                 }
-                run_loop(c, F, cheby ? LOOP_CHEBY : LOOP_PPCG, P->ppcg_inner_steps);
+                const int first_step = s.cheby_calc_steps;
+                const bool one_launch = run_loop(c, F, cheby ? LOOP_CHEBY : LOOP_PPCG, P->ppcg_inner_steps);
+                if (cheby && s.exit_reason == EXIT_PHASE) restore_residual(c, F, chunk, one_launch, first_step);
             } else if (!p_halo_fresh) {
                 // A CG iteration in Chebyshev mode (the error rose above 1 after the switch):
                 // its ext_cg_calc_w_ reads the halo of p as last refreshed before the switch,

@@ -54,6 +54,7 @@ struct SolveState {
     // test (sum r^2 <= switch_err after switch_min iterations); 0 when it does not apply.
     double switch_err;
     int switch_min;
+    int last_pass;  // iterations of the last FP64 Chebyshev pass (more than one: p went to the other buffer)
 };
 
 struct FusedArgs {
@@ -1812,6 +1813,7 @@ struct OpCheby {
         if (a.timing) return;
         SolveState& s = *a.st;
         s.par_u ^= 1;
+        s.last_pass = 1;
         if (check) s.error = rr;
         s.cheby_calc_steps = s.cheby_calc_steps + 1;
         end_iteration(a, s, PHASE_CHEBY);
@@ -1849,6 +1851,7 @@ struct OpCheby {
         SolveState& s = *a.st;
         s.par_u ^= 1;
         s.par_p ^= 1;
+        s.last_pass = nit;
         for (int k = 0; k < nit - 1; ++k) {
             s.cheby_calc_steps = s.cheby_calc_steps + 1;
             end_iteration(a, s, PHASE_CHEBY);  // cannot end the loop (pass_ok)

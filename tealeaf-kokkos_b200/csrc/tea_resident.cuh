@@ -1445,13 +1445,17 @@ __global__ void __launch_bounds__(32 * W, 1) k_res_cheby(const __grid_constant__
         }
         if (next != RN_GO) break;
     }
+    // Where CG takes over again it needs the last residual, which is not kept: the arrays stay as they
+    // were, and the host runs the iterations again by the per-call kernels (restore_residual).
+    if (P::fp32 || s.exit_reason != EXIT_PHASE) {
 #pragma unroll
-    for (int k = 0; k < RS; ++k)
-        if (t.on(k)) {
-            const Two<T> c = ld_two(t.cell(k));
-            st_cells(P::u(a), t.gidx(k), t.both(), c.x, c.y);
-            st_cells(P::p(a), t.gidx(k), t.both(), p[k][0], p[k][1]);
-        }
+        for (int k = 0; k < RS; ++k)
+            if (t.on(k)) {
+                const Two<T> c = ld_two(t.cell(k));
+                st_cells(P::u(a), t.gidx(k), t.both(), c.x, c.y);
+                st_cells(P::p(a), t.gidx(k), t.both(), p[k][0], p[k][1]);
+            }
+    }
     RES_EPILOGUE();
 }
 

@@ -169,7 +169,7 @@ STIFF_SHAPES = [(2, (5, 5)), (2, (10, 10)), (2, (16, 16)), (2, (33, 20)), (2, (2
 def test_sums_with_cancelling_terms_equal_per_call(dim, shape, dt):
     # Stiff steps: the terms of p.w are far larger than p.w.
     for seed in range(4):
-        for solver, precond in (("cg", False), ("cg", True), ("ppcg", False)):
+        for solver, precond in (("cg", False), ("cg", True), ("chebyshev", True), ("ppcg", False)):
             deck = _spec_deck(dim, shape, seed=seed, solver=solver, dt=dt, eps=1e-6, max_iters=150, presteps=20,
                               inner_steps=5, preconditioner=precond)
             _same_outcome(_outcome(deck, dim, fused=True), _outcome(deck, dim), (seed, solver, precond))
@@ -278,3 +278,23 @@ def test_waits_that_run_out_end_in_an_error_status(dim, shape, solver):
         assert np.array_equal(again[1], first[1]) and np.array_equal(again[2], first[2])
     finally:
         lib.ext_finalise_()
+
+@pytest.mark.parametrize("dim,shape", [(2, (131, 33)), (2, (127, 128)), (2, (257, 515)), (2, (860, 850)), (2, (900, 1000)),
+                                       (3, (33, 16, 5)), (3, (48, 48, 48)), (3, (66, 52, 77))])
+def test_preconditioned_chebyshev_loops_equal_per_call(dim, shape):
+    deck = _deck(dim, shape, "chebyshev", True)
+    _same(_run(deck, dim, fused=True), _run(deck, dim))
+
+
+@pytest.mark.parametrize("solver", ["chebyshev", "ppcg"])
+@pytest.mark.parametrize("dim,shape", [(2, (10, 10)), (2, (131, 33)), (2, (300, 200)), (2, (1023, 1009)), (2, (1500, 1400)),
+                                       (3, (17, 7, 9)), (3, (48, 48, 48)), (3, (101, 99, 97))])
+def test_solves_that_fall_back_to_cg_equal_per_call(dim, shape, solver):
+    # Too few CG iterations for the spectrum's bounds: the error rises above 1 again and CG goes on from the
+    # last residual.  As one launch and, without graphs, as single passes.
+    for seed, precond in ((1, False), (2, True), (3, False)):
+        deck = _spec_deck(dim, shape, seed=seed, solver=solver, dt=4.0 * (10.0 / max(shape)) ** 2, eps=1e-10,
+                          max_iters=120, presteps=4, inner_steps=4, preconditioner=precond)
+        b = _outcome(deck, dim)
+        _same_outcome(_outcome(deck, dim, fused=True), b, (seed, precond))
+        _same_outcome(_single(deck, dim, fused=True), b, (seed, precond, "single"))

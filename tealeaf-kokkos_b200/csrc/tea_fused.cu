@@ -1301,7 +1301,8 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
         R->status = TEA_ERR_BAD_ARGUMENT;
         return;
     }
-    Fused* F = ensure_fused(c, P->max_iters);
+    // The coefficient arrays take max_iters Chebyshev iterations, or all inner steps of a PPCG solve.
+    Fused* F = ensure_fused(c, solver == TEA_SOLVER_PPCG ? std::max(P->max_iters, P->ppcg_inner_steps) : P->max_iters);
     const bool cg_like = solver != TEA_SOLVER_JACOBI;
     int coefficient = P->coefficient, precond = P->preconditioner ? 1 : 0;
     double dt = P->dt;
@@ -1493,7 +1494,8 @@ TEA_EXPORT void ext_tea_leaf_solve_(const int* chunk, const tea_solve_params* P,
                     eigmax > eigmin) {
                     eigmin = eigmin * kEigMinScale;
                     eigmax = eigmax * kEigMaxScale;
-                    const int ncoef = std::min(P->max_iters + 1, F->cap);
+                    const int ncoef = std::min((ppcg_inner ? std::max(P->max_iters, P->ppcg_inner_steps) : P->max_iters) + 1,
+                                               F->cap);
                     std::vector<double> ch_a(ncoef, 0.0), ch_b(ncoef, 0.0);
                     double theta = 0.0;
                     tea_calc_ch_coefs(ch_a.data(), ch_b.data(), eigmin, eigmax, &theta, ncoef);

@@ -788,9 +788,11 @@ struct Runner {
                     if (info != 0) fail("tea_leaf: Error in calculating eigenvalues");
                     eigmin = eigmin * tea::kEigMinScale;
                     eigmax = eigmax * tea::kEigMaxScale;
-                    if ((int)ch_alphas.size() < max_cheby_iters + 1) {
-                        ch_alphas.resize(max_cheby_iters + 1, 0.0);
-                        ch_betas.resize(max_cheby_iters + 1, 0.0);
+                    // Either solver's number of coefficients, whichever is larger.
+                    const int ncoef = std::max(max_cheby_iters, use_ppcg ? cfg.tl_ppcg_inner_steps : 0) + 1;
+                    if ((int)ch_alphas.size() < ncoef) {
+                        ch_alphas.resize(ncoef, 0.0);
+                        ch_betas.resize(ncoef, 0.0);
                     }
                     if (use_cheby) {
                         tea::tea_calc_ch_coefs(ch_alphas.data(), ch_betas.data(), eigmin, eigmax, &theta,

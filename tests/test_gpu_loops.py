@@ -298,3 +298,16 @@ def test_solves_that_fall_back_to_cg_equal_per_call(dim, shape, solver):
         b = _outcome(deck, dim)
         _same_outcome(_outcome(deck, dim, fused=True), b, (seed, precond))
         _same_outcome(_single(deck, dim, fused=True), b, (seed, precond, "single"))
+
+
+@pytest.mark.parametrize("shape", [(10, 10), (131, 33), (300, 200)])
+def test_more_inner_steps_than_iterations(shape):
+    # The FP64 solve refuses inner steps beyond the iterations that are left, on both paths; no array is
+    # shorter than the steps.  The FP32 inner solve takes them all.
+    deck = _spec_deck(2, shape, seed=5, solver="ppcg", dt=0.0005 * (10.0 / max(shape)) ** 2, eps=1e-40, max_iters=14,
+                      presteps=3, inner_steps=300)
+    for kw in ({}, {"fused": True}):
+        outcome = _outcome(deck, 2, **kw)
+        assert isinstance(outcome, str) and "status 2" in outcome, outcome
+    kw = {"fused": True, "precision": tea.PRECISION_FP32_REFINED}
+    _same_outcome(_outcome(deck, 2, **kw), _single(deck, 2, **kw), shape)

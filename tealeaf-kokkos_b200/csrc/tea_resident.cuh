@@ -322,9 +322,8 @@ __device__ __forceinline__ void wide_merge(Wide& a)
         wide_add(a, b);
     }
 }
-// Over the block, by every thread; the result is valid in warp 0.  Out of line, as wide_grid: few sums
-// need it, and the on-chip loops have no registers to spare (PPCG at 1024^2 0.7 % slower with it in line).
-__device__ __noinline__ Wide wide_block(DD acc, Wide* s)
+// Over the block, by every thread; the result is valid in warp 0.
+__device__ __forceinline__ Wide wide_block(DD acc, Wide* s)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Wide a = {acc, max(res_exponent(acc.hi) - RES_E_ROOM, res_exponent(acc.lo) + RES_E_LOW)};
@@ -339,7 +338,7 @@ __device__ __noinline__ Wide wide_block(DD acc, Wide* s)
     return a;
 }
 // Over the blocks' four words each at `slots`, by one warp.
-__device__ __noinline__ Wide wide_grid(const unsigned long long* slots, int nb)
+__device__ __forceinline__ Wide wide_grid(const unsigned long long* slots, int nb)
 {
     Wide a = {{0.0, 0.0}, 0};
     for (int b = threadIdx.x & 31; b < nb; b += 32) {
@@ -349,6 +348,12 @@ __device__ __noinline__ Wide wide_grid(const unsigned long long* slots, int nb)
     wide_merge(a);
     return a;
 }
+
+// Out of line for the on-chip loops, which have no registers to spare (PPCG at 1024^2 0.7 % slower with
+// these in line), and the streamed FP64 loop (CG phase of PPCG at 256^3: the timestep 0.4 % slower in
+// line); in line for the streamed FP32 loop (CG at 256^3 0.9 % slower with calls).
+__device__ __noinline__ Wide wide_block_call(DD acc, Wide* s) { return wide_block(acc, s); }
+__device__ __noinline__ Wide wide_grid_call(const unsigned long long* slots, int nb) { return wide_grid(slots, nb); }
 
 template <bool CL = false>
 struct SumShared : ClusterShared<CL> {
@@ -364,7 +369,7 @@ struct SumShared : ClusterShared<CL> {
 enum { RN_GO = 0, RN_STOP = 1, RN_AGAIN = 2, RN_FAIL = 4 };
 
 // A block's part in the sums over the grid.
-template <bool CL = false>
+template <bool CL = false, bool CALL = false>
 struct GridSum {
     const SumArgs& sa;
     SumShared<CL>& ss;
@@ -476,7 +481,7 @@ struct GridSum {
     __device__ __forceinline__ void reduce_wide(const DD& acc, int which, C&& control)
     {
         parity ^= 1;
-        Wide s = wide_block(acc, ss.wide);
+        Wide s = CALL ? wide_block_call(acc, ss.wide) : wide_block(acc, ss.wide);
         if (warp != 0) return;
         const int nb = sa.blocks;
         if (nb > 1) {
@@ -494,7 +499,7 @@ struct GridSum {
                 }
                 counted<true>(0);
             }
-            s = wide_grid(slots, nb);
+            s = CALL ? wide_grid_call(slots, nb) : wide_grid(slots, nb);
         }
         if (lane == 0) {
             const double sum = dd_value(s.s);
@@ -626,8 +631,8 @@ struct ResShared {
 };
 
 template <class T, int RS, bool CL>
-struct ResTile : GridSum<CL> {
-    using Base = GridSum<CL>;
+struct ResTile : GridSum<CL, true> {
+    using Base = GridSum<CL, true>;
     using Base::gave_up;
     using Base::lane;
     using Base::nw;

@@ -486,7 +486,7 @@ __global__ void __launch_bounds__(ST_WARPS * 32, 1) k_stream_cg(const __grid_con
     __shared__ ResShared<false> sh;
     const FusedArgs& a = A.f;
     SolveState& s = sh.s;
-    GridSum<> sum(A.sum, sh.sum);
+    GridSum<false, !P::fp32> sum(A.sum, sh.sum);
     if (threadIdx.x == 0) {
         s = A.start ? *A.start : A.s0;
         sum.start(s.rro);

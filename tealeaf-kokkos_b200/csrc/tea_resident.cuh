@@ -46,8 +46,8 @@
 // more round through all blocks, and no more.  So a sum is the rounded sum of the threads' partials
 // except within some 2^-100 of the terms' magnitude of a rounding boundary, as it is in the per-launch
 // kernels, whose sums the tests find bit for bit.  Per cell the operations and their order are those
-// of the per-call kernels.  (Against a loop that took every sum as the limbs gave it: CG at 512^2 0.7 %
-// faster, by the compiler's schedule, PPCG at 1024^2 0.4 % and Jacobi on 33 x 150 cells 2 % slower.)
+// of the per-call kernels.  (Against a loop that took every sum as the limbs gave it: CG at 512^2 0.9 %
+// faster, by the compiler's schedule, PPCG at 1024^2 the same, Jacobi on 33 x 150 cells 1.7 % slower.)
 //
 // Clusters.  Up to 16 blocks with one row a warp (some 16000 cells) form one cluster: limbs and rim
 // values go straight into the other blocks' shared memory, and an mbarrier there counts their
@@ -407,10 +407,10 @@ struct GridSum {
     __device__ __forceinline__ int reduce(const DD& acc, int which, M&& meanwhile, C&& control, N&& after)
     {
         const int E = ss.scale[which];
-        int v[RES_LIMBS];
-        res_limbs(acc.hi, acc.lo, E, v);  // whatever they are for a partial out of range: the flag says so
         if (max(res_exponent(acc.hi) - RES_E_ROOM, res_exponent(acc.lo) + RES_E_LOW) > E)
             atomicOr(&ss.bad, isfinite(acc.hi) ? 1 : 2);
+        int v[RES_LIMBS];
+        res_limbs(acc.hi, acc.lo, E, v);  // whatever they are for a partial out of range: the flag says so
 #pragma unroll
         for (int i = 0; i < RES_LIMBS; ++i) v[i] = __reduce_add_sync(0xffffffffu, v[i]);
         if (lane == 0) {
@@ -421,6 +421,7 @@ struct GridSum {
         __syncthreads();
         if (warp == 0) {
             unsigned bad = ss.bad;
+            const int lift = ss.lift[which];
             long long tot[RES_LIMBS];
 #pragma unroll
             for (int i = 0; i < RES_LIMBS; ++i) {
@@ -454,9 +455,9 @@ struct GridSum {
                 const bool doubtful = (s.hi + (low + slack)) != (s.hi + (low - slack));
                 int next = RN_AGAIN;
                 if (__builtin_expect(!doubtful && bad == 0, 1)) {
-                    next = control(sum) ? RN_GO : RN_STOP;
-                    ss.scale[which] = res_clamp(res_exponent(sum) + ss.lift[which]);
+                    ss.scale[which] = res_clamp(res_exponent(sum) + lift);
                     ss.sum = sum;
+                    next = control(sum) ? RN_GO : RN_STOP;
                 } else if (bad & 2) {  // as the double-double merges make of it
                     next = control(CUDART_NAN) ? RN_GO : RN_STOP;
                     ss.sum = CUDART_NAN;
